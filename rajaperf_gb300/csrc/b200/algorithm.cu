@@ -14,6 +14,7 @@
 #include "b200_internal.cuh"
 #include "b200_fma_form.cuh"
 #include "b200_async.cuh"
+#include "b200_launch.cuh"
 #include "b200_lookback.cuh"
 #include "b200_pipeline.cuh"
 #include "b200_reduce.cuh"
@@ -428,11 +429,11 @@ int launch_scan(const char* name, const T* x, T* y, int64_t n, T init, void* ws,
 // ---- REDUCE_SUM -------------------------------------------------------------
 template <int BS, int IT>
 __global__ void __launch_bounds__(BS)
-reduce_sum_kernel(const double* __restrict__ x, int64_t n, double init,
-                  double* __restrict__ out, double* __restrict__ partials,
-                  unsigned int* __restrict__ counter, int zero) {
+reduce_sum_kernel(const double* x, int64_t n, double init, double* out, double* partials,
+                  unsigned int* counter, int zero) {
   __shared__ double smem[BS / 32];
   __shared__ bool last_flag;
+  const int64_t first = begin() + threadIdx.x;
   double s = 0.0;
   // s + v as a register-operand FMA (fform: bit-identical, full FP64 rate
   // where DADD gets 5/6 of it); `zero` is 0 at run time
@@ -442,8 +443,8 @@ reduce_sum_kernel(const double* __restrict__ x, int64_t n, double init,
     double v[IT];
 #pragma unroll
     for (int u = 0; u < IT; ++u) {
-      int64_t i = t0 + u * BS + threadIdx.x;
-      v[u] = (i < n) ? __ldg(x + i) : 0.0;
+      const int64_t i = t0 + u * BS + first;
+      v[u] = (i < n) ? x[i] : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < IT; ++u) s = fma(v[u], one, s);  // s + v[u]
@@ -506,7 +507,8 @@ int b200_algorithm_reduce_sum(const double* x, int64_t n, double sum_init, doubl
   double* partials = reinterpret_cast<double*>(static_cast<char*>(workspace) + 256);
   cudaStream_t st = as_stream(stream);
   B200_DISPATCH_BLOCK(block, BS, B200_DISPATCH_ITEMS(items, IT,
-    reduce_sum_kernel<BS, IT><<<grid, BS, 0, st>>>(x, n, sum_init, sum, partials, counter, 0)));
+    launch(reduce_sum_kernel<BS, IT>, grid, BS, 0, st, x, n, sum_init, sum, partials, counter,
+           0)));
   return after_launch("b200_algorithm_reduce_sum");
 }
 

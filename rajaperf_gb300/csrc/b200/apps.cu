@@ -16,24 +16,28 @@ namespace {
 
 // apps/PRESSURE.hpp:39-46 (BODY1 then BODY2)
 struct Pressure {
-  const double* __restrict__ compression;
-  double* __restrict__ bvc;
-  double* __restrict__ p_new;
-  const double* __restrict__ e_old;
-  const double* __restrict__ vnewc;
+  const double* compression;
+  double* bvc;
+  double* p_new;
+  const double* e_old;
+  const double* vnewc;
   double cls, p_cut, pmin, eosvmax;
   int zero;  // 0 at run time (fform)
-  __device__ void operator()(int64_t i) const {
+  struct Out { double bvc, p; };
+  __device__ Out compute(int64_t i) const {
     // the add and the two products as register-operand FMAs (fform,
     // bit-identical), the FP64 pipe's full-rate form
     const fform::Regs fr = fform::regs(zero);
     const double b = fform::mul(fform::reg(cls, zero), fform::add(ld(compression + i), fr.one, fr), fr);
-    bvc[i] = b;
     double p = fform::mul(b, ld(e_old + i), fr);
     if (fabs(p) < p_cut) p = 0.0;
     if (ld(vnewc + i) >= eosvmax) p = 0.0;
     if (p < pmin) p = pmin;
-    p_new[i] = p;
+    return {b, p};
+  }
+  __device__ void store(int64_t i, const Out& v) const {
+    bvc[i] = v.bvc;
+    p_new[i] = v.p;
   }
 };
 
@@ -41,21 +45,21 @@ struct Pressure {
 // the exact power-of-two products and the division by 6.0 move to the
 // integer and FP32 pipes (see body()).
 struct Energy {
-  double* __restrict__ e_new;
-  const double* __restrict__ e_old;
-  const double* __restrict__ delvc;
-  const double* __restrict__ p_new;
-  const double* __restrict__ p_old;
-  double* __restrict__ q_new;
-  const double* __restrict__ q_old;
-  const double* __restrict__ work;
-  const double* __restrict__ compHalfStep;
-  const double* __restrict__ pHalfStep;
-  const double* __restrict__ bvc;
-  const double* __restrict__ pbvc;
-  const double* __restrict__ ql_old;
-  const double* __restrict__ qq_old;
-  const double* __restrict__ vnewc;
+  double* e_new;
+  const double* e_old;
+  const double* delvc;
+  const double* p_new;
+  const double* p_old;
+  double* q_new;
+  const double* q_old;
+  const double* work;
+  const double* compHalfStep;
+  const double* pHalfStep;
+  const double* bvc;
+  const double* pbvc;
+  const double* ql_old;
+  const double* qq_old;
+  const double* vnewc;
   double rho0, e_cut, emin, q_cut;
 
   // One element, BODY1..BODY6.  FAST: the power-of-two products (0.5 * dv,
@@ -63,8 +67,10 @@ struct Energy {
   // f64emu::div_fast -- all exact or correctly rounded, so every result bit
   // equals the FP64 pipe's -- and `slow` reports an operand outside their
   // fast paths, for which the caller recomputes the element natively.
+  static constexpr bool kOneByOne = true;
+  struct Out { double e, q; };
   template <bool FAST>
-  __device__ __forceinline__ void body(int64_t i, bool& slow) const {
+  __device__ __forceinline__ Out body(int64_t i, bool& slow) const {
     const double dv = ld(delvc + i);
     const double po = ld(p_old + i), qo = ld(q_old + i), wk = ld(work + i);
     const double ph = ld(pHalfStep + i), pn = ld(p_new + i);
@@ -117,13 +123,17 @@ struct Energy {
       qn = (ssc * ld(ql_old + i) + ld(qq_old + i));
       if (fabs(qn) < q_cut) qn = 0.0;
     }
-    e_new[i] = e;
-    q_new[i] = qn;
+    return {e, qn};
   }
-  __device__ void operator()(int64_t i) const {
+  __device__ Out compute(int64_t i) const {
     bool slow = false;
-    body<true>(i, slow);
-    if (__any_sync(__activemask(), slow) && slow) body<false>(i, slow);
+    Out v = body<true>(i, slow);
+    if (__any_sync(__activemask(), slow) && slow) v = body<false>(i, slow);
+    return v;
+  }
+  __device__ void store(int64_t i, const Out& v) const {
+    e_new[i] = v.e;
+    q_new[i] = v.q;
   }
 };
 
@@ -132,13 +142,14 @@ struct Energy {
 // from NDPTRSET (apps/AppsData.hpp: v0=v, v1=v0+1, v2=v0+jp, v3=v1+jp,
 // v4..v7 = v0..v3 + kp).
 struct Vol3D {
-  const double* __restrict__ x;
-  const double* __restrict__ y;
-  const double* __restrict__ z;
-  double* __restrict__ vol;
+  const double* x;
+  const double* y;
+  const double* z;
+  double* vol;
   double vnormq;
   int64_t jp, kp, ibegin;
-  __device__ void operator()(int64_t ii) const {
+  using Out = double;
+  __device__ Out compute(int64_t ii) const {
     const int64_t i = ibegin + ii;
     const int64_t o1 = 1, o2 = jp, o3 = 1 + jp, o4 = kp, o5 = 1 + kp, o6 = jp + kp,
                   o7 = 1 + jp + kp;
@@ -177,8 +188,9 @@ struct Vol3D {
     czx = z71 * x50 - x71 * z50;
     cxy = x71 * y50 - y71 * x50;
     v += xps * cyz + yps * czx + zps * cxy;
-    vol[i] = v * vnormq;
+    return v * vnormq;
   }
+  __device__ void store(int64_t ii, Out v) const { vol[ibegin + ii] = v; }
 };
 
 // apps/DEL_DOT_VEC_2D.hpp:65-90 with corners from NDSET2D (AppsData.hpp:
@@ -195,12 +207,12 @@ struct Vol3D {
 // integer pipes (f64emu::add_close_fast, bit-identical).
 template <bool HALF_POW2, int KD = 0>
 struct DelDotVec2D {
-  const double* __restrict__ x;
-  const double* __restrict__ y;
-  const double* __restrict__ xdot;
-  const double* __restrict__ ydot;
-  double* __restrict__ div;
-  const int64_t* __restrict__ real_zones;
+  const double* x;
+  const double* y;
+  const double* xdot;
+  const double* ydot;
+  double* div;
+  const int64_t* real_zones;
   int64_t jp;
   double ptiny, half;
   int zero;  // 0 at run time (fform)
@@ -284,7 +296,9 @@ struct DelDotVec2D {
                           fform::add(fform::add(fform::add(y1, y2, fr), y3, fr), y4, fr);
     return fform::add(fform::add(dfxdx, dfydy, fr), affine, fr);
   }
-  __device__ void operator()(int64_t ii) const {
+  static constexpr bool kOneByOne = true;
+  struct Out { int64_t zone; double div; };
+  __device__ Out compute(int64_t ii) const {
     const int64_t i = ld(real_zones + ii);
     const int64_t c1 = i + 1, c2 = i + 1 + jp, c3 = i + jp, c4 = i;
     const double x1 = ld(x + c1), x2 = ld(x + c2), x3 = ld(x + c3), x4 = ld(x + c4);
@@ -300,8 +314,9 @@ struct DelDotVec2D {
       if (slow)
         r = body(x1, x2, x3, x4, y1, y2, y3, y4, fx1, fx2, fx3, fx4, fy1, fy2, fy3, fy4,
                  false, slow);
-    div[i] = r;
+    return {i, r};
   }
+  __device__ void store(int64_t, const Out& v) const { div[v.zone] = v.div; }
 };
 
 }  // namespace
@@ -371,7 +386,7 @@ int b200_apps_del_dot_vec_2d(const double* x, const double* y, const double* xdo
     auto go = [&](auto f) -> int {
       if (n_real_zones <= 0) return B200_OK;
       const Shape sh = resolve_1d(nullptr, n_real_zones, 256, 2, 1);
-      map_kernel<256, 2, decltype(f)><<<sh.grid, 256, 0, as_stream(stream)>>>(f, n_real_zones);
+      launch(map_kernel<256, 2, decltype(f)>, sh.grid, 256, 0, as_stream(stream), f, n_real_zones);
       return after_launch("b200_apps_del_dot_vec_2d");
     };
     switch (kd) {

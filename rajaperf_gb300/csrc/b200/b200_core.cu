@@ -98,6 +98,12 @@ int allow_dynamic_smem(const void* kernel, size_t bytes, const char* what) {
   return B200_OK;
 }
 
+int spread(int64_t units, int block, int items) {
+  const int64_t want = 2 * static_cast<int64_t>(device_info().sm_count);
+  while (items > 1 && ceil_div(units, static_cast<int64_t>(block) * items) < want) items /= 2;
+  return items;
+}
+
 Shape resolve_1d(const b200_tune* t, int64_t units, int def_block,
                  int def_items, int def_vec, int64_t max_grid) {
   Shape s;

@@ -69,6 +69,11 @@ struct Shape {
 Shape resolve_1d(const b200_tune* t, int64_t units, int def_block,
                  int def_items, int def_vec, int64_t max_grid = 0);
 
+// Default items per thread for `units` work items: `items`, halved until the
+// tiles give every SM two CTAs (or one item per thread), so that a short
+// array spreads over the chip instead of queueing in a few CTAs' threads.
+int spread(int64_t units, int block, int items);
+
 // Limit of the bounded device-side waits of a call (b200_tune.wait_limit_us;
 // 0 or negative = `def_ns`).
 inline uint64_t wait_limit_ns(const b200_tune* t, uint64_t def_ns) {

@@ -145,7 +145,7 @@ __device__ __forceinline__ KeyLoc block_keyloc(KeyLoc v, KeyLoc* smem) {
 }
 
 // Publishes this CTA's partial and reports whether this CTA arrived last.
-// Thread 0 must call it; the result is broadcast through `flag`.
+// Every thread calls it; the result is broadcast through `flag`.
 __device__ __forceinline__ bool arrive_last(unsigned int* counter,
                                             bool* flag) {
   if (threadIdx.x == 0) {

@@ -9,21 +9,24 @@ namespace {
 
 // basic/DAXPY.hpp: y[i] += a * x[i]
 struct Daxpy {
-  double* __restrict__ y;
-  const double* __restrict__ x;
+  double* y;
+  const double* x;
   double a;
-  __device__ void operator()(int64_t i) const { y[i] += a * ld(x + i); }
+  using Out = double;
+  __device__ Out compute(int64_t i) const { return y[i] + a * ld(x + i); }
+  __device__ void store(int64_t i, Out v) const { y[i] = v; }
 };
 
 // basic/INIT3.hpp: out1 = out2 = out3 = -in1 - in2
 struct Init3 {
-  double* __restrict__ out1;
-  double* __restrict__ out2;
-  double* __restrict__ out3;
-  const double* __restrict__ in1;
-  const double* __restrict__ in2;
-  __device__ void operator()(int64_t i) const {
-    const double v = -ld(in1 + i) - ld(in2 + i);
+  double* out1;
+  double* out2;
+  double* out3;
+  const double* in1;
+  const double* in2;
+  using Out = double;
+  __device__ Out compute(int64_t i) const { return -ld(in1 + i) - ld(in2 + i); }
+  __device__ void store(int64_t i, Out v) const {
     out3[i] = v;
     out2[i] = v;
     out1[i] = v;
@@ -32,16 +35,20 @@ struct Init3 {
 
 // basic/MULADDSUB.hpp
 struct MulAddSub {
-  double* __restrict__ out1;
-  double* __restrict__ out2;
-  double* __restrict__ out3;
-  const double* __restrict__ in1;
-  const double* __restrict__ in2;
-  __device__ void operator()(int64_t i) const {
+  double* out1;
+  double* out2;
+  double* out3;
+  const double* in1;
+  const double* in2;
+  struct Out { double product, sum, difference; };
+  __device__ Out compute(int64_t i) const {
     const double a = ld(in1 + i), b = ld(in2 + i);
-    out1[i] = a * b;
-    out2[i] = a + b;
-    out3[i] = a - b;
+    return {a * b, a + b, a - b};
+  }
+  __device__ void store(int64_t i, const Out& o) const {
+    out1[i] = o.product;
+    out2[i] = o.sum;
+    out3[i] = o.difference;
   }
 };
 

@@ -18,17 +18,19 @@ namespace {
 // product r * z as an FMA with -0, the coefficients in per-thread registers),
 // which the FP64 pipe issues at its full rate; `zero` is 0 at run time.
 struct Hydro1D {
-  double* __restrict__ x;
-  const double* __restrict__ y;
-  const double* __restrict__ z;
+  double* x;
+  const double* y;
+  const double* z;
   double q, r, t;
   int zero;
-  __device__ void operator()(int64_t i) const {
+  using Out = double;
+  __device__ Out compute(int64_t i) const {
     const fform::Regs fr = fform::regs(zero);
-    x[i] = fma(ld(y + i), fma(fform::reg(t, zero), ld(z + i + 11),
+    return fma(ld(y + i), fma(fform::reg(t, zero), ld(z + i + 11),
                               fform::mul(fform::reg(r, zero), ld(z + i + 10), fr)),
                fform::reg(q, zero));
   }
+  __device__ void store(int64_t i, Out v) const { x[i] = v; }
 };
 
 // lcals/EOS.hpp:33: x = u + r (z + r y) + t (u3 + r (u2 + r u1) + t (u6 +
@@ -36,19 +38,21 @@ struct Hydro1D {
 // q, r, t in per-thread registers (fform::reg) so that every FMA has
 // register operands; `zero` is 0 at run time.
 struct Eos {
-  double* __restrict__ x;
-  const double* __restrict__ y;
-  const double* __restrict__ z;
-  const double* __restrict__ u;
+  double* x;
+  const double* y;
+  const double* z;
+  const double* u;
   double q, r, t;
   int zero;
-  __device__ void operator()(int64_t i) const {
+  using Out = double;
+  __device__ Out compute(int64_t i) const {
     const double rr = fform::reg(r, zero), tr = fform::reg(t, zero), qr = fform::reg(q, zero);
     const double a = fma(rr, fma(rr, ld(y + i), ld(z + i)), ld(u + i));
     const double b = fma(rr, fma(rr, ld(u + i + 1), ld(u + i + 2)), ld(u + i + 3));
     const double c = fma(qr, fma(qr, ld(u + i + 4), ld(u + i + 5)), ld(u + i + 6));
-    x[i] = fma(tr, fma(tr, c, b), a);
+    return fma(tr, fma(tr, c, b), a);
   }
+  __device__ void store(int64_t i, Out v) const { x[i] = v; }
 };
 
 // Element map with part of each element's FP64 work on the integer pipes.
@@ -63,26 +67,32 @@ struct Eos {
 template <int BS, int PT, class F>
 __global__ void __launch_bounds__(BS) split_map_kernel(F f, int64_t n) {
   static_assert(PT >= 1 && PT <= 64, "one redo bit per element");
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * BS * PT + threadIdx.x + begin();
   const auto rg = f.regs();
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * BS * PT + threadIdx.x;
   uint64_t redo = 0;
+  double v[PT];
   auto element = [&](int p) {
-    const int64_t i = base + static_cast<int64_t>(p) * BS;
     bool slow = false;
-    const double v = f.split(i, rg, slow);
-    if (!slow) f.store(i, v);
-    else redo |= 1ull << p;
+    v[p] = f.split(base + static_cast<int64_t>(p) * BS, rg, slow);
+    if (slow) redo |= 1ull << p;
+  };
+  auto store = [&](int p) {
+    if (!((redo >> p) & 1u)) f.store(base + static_cast<int64_t>(p) * BS, v[p]);
   };
   if (static_cast<int64_t>(blockIdx.x + 1) * BS * PT <= n) {
     // a whole CTA in range: no bounds test, so the unrolled elements' loads
     // issue together
 #pragma unroll
     for (int p = 0; p < PT; ++p) element(p);
+#pragma unroll
+    for (int p = 0; p < PT; ++p) store(p);
   } else {
-    for (int p = 0; p < PT; ++p) {
-      if (base + static_cast<int64_t>(p) * BS >= n) break;
-      element(p);
-    }
+#pragma unroll
+    for (int p = 0; p < PT; ++p)
+      if (base + static_cast<int64_t>(p) * BS < n) element(p);
+#pragma unroll
+    for (int p = 0; p < PT; ++p)
+      if (base + static_cast<int64_t>(p) * BS < n) store(p);
   }
   if (__any_sync(__activemask(), redo != 0)) {
     for (int p = 0; p < PT; ++p) {
@@ -97,10 +107,10 @@ __global__ void __launch_bounds__(BS) split_map_kernel(F f, int64_t n) {
 // three outer ones of each group, then the two in t.
 template <int KF>
 struct EosSplit {
-  double* __restrict__ x;
-  const double* __restrict__ y;
-  const double* __restrict__ z;
-  const double* __restrict__ u;
+  double* x;
+  const double* y;
+  const double* z;
+  const double* u;
   double q, r, t;
   int zero;
   struct Regs { double q, r, t; };
@@ -135,8 +145,8 @@ int launch_split_map(const char* name, const F& f, int64_t n, int bs, int pt, cu
   const int64_t grid = ceil_div(n, static_cast<int64_t>(bs) * pt);
   if (grid > 0x7fffffff) return invalid("%s: n too large", name);
   auto go = [&](auto B, auto P) {
-    split_map_kernel<decltype(B)::value, decltype(P)::value, F>
-        <<<static_cast<unsigned>(grid), decltype(B)::value, 0, st>>>(f, n);
+    launch(split_map_kernel<decltype(B)::value, decltype(P)::value, F>,
+           static_cast<unsigned>(grid), decltype(B)::value, 0, st, f, n);
   };
   auto by_pt = [&](auto B) {
     switch (pt) {
@@ -154,9 +164,11 @@ int launch_split_map(const char* name, const F& f, int64_t n, int bs, int pt, cu
 
 // lcals/FIRST_DIFF.hpp:25
 struct FirstDiff {
-  double* __restrict__ x;
-  const double* __restrict__ y;
-  __device__ void operator()(int64_t i) const { x[i] = ld(y + i + 1) - ld(y + i); }
+  double* x;
+  const double* y;
+  using Out = double;
+  __device__ Out compute(int64_t i) const { return ld(y + i + 1) - ld(y + i); }
+  __device__ void store(int64_t i, Out v) const { x[i] = v; }
 };
 
 // lcals/INT_PREDICT.hpp:40 -- px[0..n) is written, planes 2..12 are read.
@@ -166,7 +178,9 @@ struct IntPredict {
   double dm22, dm23, dm24, dm25, dm26, dm27, dm28, c0;
   // The first product runs on the integer pipe (f64emu::mul_fast, correctly
   // rounded); the rest of the sum contracts into FMAs on the FP64 pipe.
-  __device__ void operator()(int64_t i) const {
+  static constexpr bool kOneByOne = true;
+  using Out = double;
+  __device__ Out compute(int64_t i) const {
     const double* p = px;
     const double p12 = ld(p + i + o * 12);
     bool slow = false;
@@ -182,68 +196,50 @@ struct IntPredict {
           dm24 * ld(p + i + o * 8) + dm23 * ld(p + i + o * 7) +
           dm22 * ld(p + i + o * 6) +
           c0 * (ld(p + i + o * 4) + ld(p + i + o * 5)) + ld(p + i + o * 2);
-    px[i] = v;
+    return v;
   }
+  __device__ void store(int64_t i, Out v) const { px[i] = v; }
 };
 
 // lcals/DIFF_PREDICT.hpp -- planes 4..13 of px are updated in place per i.
 struct DiffPredict {
   double* px;
-  const double* __restrict__ cx;
+  const double* cx;
   int64_t o;
   // The suite reads each plane of px before overwriting it and never reads
   // it again, and for o = n >= 1 the planes are disjoint: so all ten loads
   // are issued first (independent, in flight together) and the ten stores
   // follow.  The same differences, in the same order, as the macro.
-  __device__ void operator()(int64_t i) const {
+  static constexpr bool kOneByOne = true;
+  struct Out { double q[10]; };
+  __device__ Out compute(int64_t i) const {
     double p[9];  // planes 4..12 before the update
 #pragma unroll
     for (int k = 0; k < 9; ++k) p[k] = px[i + o * (4 + k)];
-    double ar, br, cr;
-    double q4, q5, q6, q7, q8, q9, q10, q11, q12, q13;
-    ar = ld(cx + i + o * 4);
-    br = ar - p[0];
-    q4 = ar;
-    cr = br - p[1];
-    q5 = br;
-    ar = cr - p[2];
-    q6 = cr;
-    br = ar - p[3];
-    q7 = ar;
-    cr = br - p[4];
-    q8 = br;
-    ar = cr - p[5];
-    q9 = cr;
-    br = ar - p[6];
-    q10 = ar;
-    cr = br - p[7];
-    q11 = br;
-    q13 = cr - p[8];
-    q12 = cr;
-    px[i + o * 4] = q4;
-    px[i + o * 5] = q5;
-    px[i + o * 6] = q6;
-    px[i + o * 7] = q7;
-    px[i + o * 8] = q8;
-    px[i + o * 9] = q9;
-    px[i + o * 10] = q10;
-    px[i + o * 11] = q11;
-    px[i + o * 12] = q12;
-    px[i + o * 13] = q13;
+    Out r;
+    r.q[0] = ld(cx + i + o * 4);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) r.q[k + 1] = r.q[k] - p[k];
+    return r;
+  }
+  __device__ void store(int64_t i, const Out& r) const {
+#pragma unroll
+    for (int k = 0; k < 10; ++k) px[i + o * (4 + k)] = r.q[k];
   }
 };
 
 // lcals/PLANCKIAN.hpp
 struct Planckian {
-  const double* __restrict__ x;
-  double* __restrict__ y;
-  const double* __restrict__ u;
-  const double* __restrict__ v;
-  double* __restrict__ w;
+  const double* x;
+  double* y;
+  const double* u;
+  const double* v;
+  double* w;
   // The two divisions run on the integer and FP32 pipes (f64emu::div_fast,
   // correctly rounded); an element with an operand or quotient outside its
   // fast path (zero, subnormal, non-finite) is recomputed natively.
-  __device__ void operator()(int64_t i) const {
+  struct Out { double y, w; };
+  __device__ Out compute(int64_t i) const {
     bool slow = false;
     const double ui = ld(u + i), vi = ld(v + i), xi = ld(x + i);
     double yi = f64emu::div_fast(ui, vi, slow);
@@ -252,8 +248,11 @@ struct Planckian {
       yi = ui / vi;
       wi = xi / (exp(yi) - 1.0);
     }
-    y[i] = yi;
-    w[i] = wi;
+    return {yi, wi};
+  }
+  __device__ void store(int64_t i, const Out& v) const {
+    y[i] = v.y;
+    w[i] = v.w;
   }
 };
 
@@ -263,11 +262,9 @@ struct Planckian {
 // launches instead of three and zu/zv are not re-read for BODY3.
 template <int BS>
 __global__ void __launch_bounds__(BS)
-hydro2d_body1(double* __restrict__ za, double* __restrict__ zb,
-              const double* __restrict__ zm, const double* __restrict__ zp,
-              const double* __restrict__ zq, const double* __restrict__ zr,
-              int64_t kn, int64_t jn, int zero) {
-  const int64_t j = 1 + static_cast<int64_t>(blockIdx.x) * BS + threadIdx.x;
+hydro2d_body1(double* za, double* zb, const double* zm, const double* zp, const double* zq,
+              const double* zr, int64_t kn, int64_t jn, int zero) {
+  const int64_t j = 1 + begin() + static_cast<int64_t>(blockIdx.x) * BS + threadIdx.x;
   if (j >= jn - 1) return;
   // The two divisions and the two products run on the integer and FP32
   // pipes (f64emu::div_fast and f64emu::mul_fast, correctly rounded,
@@ -280,19 +277,21 @@ hydro2d_body1(double* __restrict__ za, double* __restrict__ zb,
   bool slow = false;
   for (int64_t k = 1 + blockIdx.y; k < kn - 1; k += gridDim.y) {
     const int64_t c = j + k * jn;
-    za[c] = f64emu::div_fast(
+    const double a = f64emu::div_fast(
         f64emu::mul_fast(
             fform::sub(fform::sub(fform::add(ld(zp + c - 1 + jn), ld(zq + c - 1 + jn), fr),
                                   ld(zp + c - 1), fr),
                        ld(zq + c - 1), fr),
             fform::add(ld(zr + c), ld(zr + c - 1), fr), slow),
         fform::add(ld(zm + c - 1), ld(zm + c - 1 + jn), fr), slow);
-    zb[c] = f64emu::div_fast(
+    const double b = f64emu::div_fast(
         f64emu::mul_fast(
             fform::sub(fform::sub(fform::add(ld(zp + c - 1), ld(zq + c - 1), fr), ld(zp + c), fr),
                        ld(zq + c), fr),
             fform::add(ld(zr + c), ld(zr + c - jn), fr), slow),
         fform::add(ld(zm + c), ld(zm + c - 1), fr), slow);
+    za[c] = a;
+    zb[c] = b;
   }
   if (__any_sync(__activemask(), slow) && slow) {
     for (int64_t k = 1 + blockIdx.y; k < kn - 1; k += gridDim.y) {
@@ -314,13 +313,11 @@ hydro2d_body1(double* __restrict__ za, double* __restrict__ zb,
 // predicated FP64 instructions, which occupy the FP64 pipe in every warp.
 template <int BS, int KH>
 __global__ void __launch_bounds__(BS)
-hydro2d_body23(const double* __restrict__ za, const double* __restrict__ zb,
-               const double* __restrict__ zr, double* __restrict__ zu,
-               double* __restrict__ zv, const double* __restrict__ zz,
-               double* __restrict__ zrout, double* __restrict__ zzout, double s,
-               double t, int64_t kn, int64_t jn, int zero) {
+hydro2d_body23(const double* za, const double* zb, const double* zr, double* zu, double* zv,
+               const double* zz, double* zrout, double* zzout, double s, double t, int64_t kn,
+               int64_t jn, int zero) {
   static_assert(KH >= 0 && KH <= 8, "0..8 integer-pipe differences");
-  const int64_t j = 1 + static_cast<int64_t>(blockIdx.x) * BS + threadIdx.x;
+  const int64_t j = 1 + begin() + static_cast<int64_t>(blockIdx.x) * BS + threadIdx.x;
   if (j >= jn - 1) return;
   const unsigned live = __activemask();
   // Every FP64 instruction a register-operand FMA (fform: the differences and
@@ -380,12 +377,12 @@ hydro2d_body23(const double* __restrict__ za, const double* __restrict__ zb,
 // (order_key), which order exactly as '<' on the doubles.
 template <int BS, int IT, bool VEC>
 __global__ void __launch_bounds__(BS)
-first_min_kernel(const double* __restrict__ x, int64_t n, double xmin_init,
-                 int64_t initloc, int64_t* __restrict__ minloc_out,
-                 double* __restrict__ minval_out, KeyLoc* __restrict__ partials,
-                 unsigned int* __restrict__ counter) {
+first_min_kernel(const double* x, int64_t n, double xmin_init, int64_t initloc,
+                 int64_t* minloc_out, double* minval_out, KeyLoc* partials,
+                 unsigned int* counter) {
   __shared__ KeyLoc smem[BS / 32];
   __shared__ bool last_flag;
+  const int64_t first = begin() + threadIdx.x;
   const long long* xb = reinterpret_cast<const long long*>(x);
   // A NaN initial value is never beaten by a strict '<' scan: give it the
   // smallest key so that nothing compares less.
@@ -412,12 +409,12 @@ first_min_kernel(const double* __restrict__ x, int64_t n, double xmin_init,
       longlong2 v[IT];
 #pragma unroll
       for (int u = 0; u < IT; ++u) {
-        const int64_t iv = t0 + u * BS + threadIdx.x;
-        v[u] = (iv < nv) ? __ldg(xv + iv) : make_longlong2(0LL, 0LL);
+        const int64_t iv = t0 + u * BS + first;
+        v[u] = (iv < nv) ? xv[iv] : make_longlong2(0LL, 0LL);
       }
 #pragma unroll
       for (int u = 0; u < IT; ++u) {
-        const int64_t iv = t0 + u * BS + threadIdx.x;
+        const int64_t iv = t0 + u * BS + first;
         if (iv < nv && (maybe(v[u].x) || maybe(v[u].y))) {
           const long long k0 = order_key(v[u].x), k1 = order_key(v[u].y);
           if (k0 < m.key) { m.key = k0; m.loc = 2 * iv; }
@@ -426,8 +423,8 @@ first_min_kernel(const double* __restrict__ x, int64_t n, double xmin_init,
         }
       }
     }
-    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {  // odd tail element
-      const long long k = order_key(__ldg(xb + n - 1));
+    if ((n & 1) && blockIdx.x == 0 && first == 0) {  // odd tail element
+      const long long k = order_key(xb[n - 1]);
       if (k < m.key) { m.key = k; m.loc = n - 1; }
     }
   } else {
@@ -436,12 +433,12 @@ first_min_kernel(const double* __restrict__ x, int64_t n, double xmin_init,
       long long v[IT];
 #pragma unroll
       for (int u = 0; u < IT; ++u) {
-        int64_t i = t0 + u * BS + threadIdx.x;
-        v[u] = (i < n) ? __ldg(xb + i) : 0LL;
+        int64_t i = t0 + u * BS + first;
+        v[u] = (i < n) ? xb[i] : 0LL;
       }
 #pragma unroll
       for (int u = 0; u < IT; ++u) {
-        int64_t i = t0 + u * BS + threadIdx.x;
+        int64_t i = t0 + u * BS + first;
         if (i < n && maybe(v[u])) {
           long long k = order_key(v[u]);
           if (k < m.key) { m.key = k; m.loc = i; }
@@ -588,10 +585,10 @@ int b200_lcals_hydro_2d(double* za, double* zb, const double* zm, const double* 
   if (kh < 0 || kh > 8 || (kh & 1)) return invalid("b200_lcals_hydro_2d: bad tile_z");
   if (ceil_div(kn - 2, static_cast<int64_t>(grid.y)) > 64) kh = 0;  // one redo bit per point
   B200_DISPATCH_BLOCK(bs, BS,
-    hydro2d_body1<BS><<<grid, BS, 0, st>>>(za, zb, zm, zp, zq, zr, kn, jn, 0);
+    launch(hydro2d_body1<BS>, grid, BS, 0, st, za, zb, zm, zp, zq, zr, kn, jn, 0);
     auto body23 = [&](auto K) {
-      hydro2d_body23<BS, decltype(K)::value><<<grid, BS, 0, st>>>(za, zb, zr, zu, zv, zz, zrout,
-                                                                  zzout, s, t, kn, jn, 0);
+      launch(hydro2d_body23<BS, decltype(K)::value>, grid, BS, 0, st, za, zb, zr, zu, zv, zz,
+             zrout, zzout, s, t, kn, jn, 0);
     };
     switch (kh) {
       case 0: body23(std::integral_constant<int, 0>{}); break;
@@ -624,12 +621,12 @@ int b200_lcals_first_min(const double* x, int64_t n, double xmin_init, int64_t i
   cudaStream_t st = as_stream(stream);
   if (vec) {
     B200_DISPATCH_BLOCK(block, BS, B200_DISPATCH_ITEMS(items, IT,
-      first_min_kernel<BS, IT, true><<<grid, BS, 0, st>>>(x, n, xmin_init, initloc, minloc,
-                                                          minval, partials, counter)));
+      launch(first_min_kernel<BS, IT, true>, grid, BS, 0, st, x, n, xmin_init, initloc, minloc,
+             minval, partials, counter)));
   } else {
     B200_DISPATCH_BLOCK(block, BS, B200_DISPATCH_ITEMS(items, IT,
-      first_min_kernel<BS, IT, false><<<grid, BS, 0, st>>>(x, n, xmin_init, initloc, minloc,
-                                                           minval, partials, counter)));
+      launch(first_min_kernel<BS, IT, false>, grid, BS, 0, st, x, n, xmin_init, initloc, minloc,
+             minval, partials, counter)));
   }
   return after_launch("b200_lcals_first_min");
 }

@@ -6,6 +6,7 @@
 // is one tile per CTA (the hardware scheduler balances the tail); arrays that
 // are not 16-byte aligned take the scalar path with the same shape.
 #include "b200_internal.cuh"
+#include "b200_launch.cuh"
 #include "b200_reduce.cuh"
 
 using namespace b200;
@@ -21,102 +22,66 @@ constexpr int kItems = 4;
        t0 < (UNITS);                                                          \
        t0 += static_cast<int64_t>(gridDim.x) * (BS * IT))
 
-template <typename T>
-__device__ __forceinline__ T ldg(const T* p) { return __ldg(p); }
+// One element-wise body per kernel: out[i] = f(in1[i], in2[i]) (COPY and MUL
+// read one array).
+struct CopyOp {
+  static constexpr int kInputs = 1;
+  __device__ double operator()(double a, double) const { return a; }
+};
+struct MulOp {
+  static constexpr int kInputs = 1;
+  double alpha;
+  __device__ double operator()(double c, double) const { return alpha * c; }
+};
+struct AddOp {
+  static constexpr int kInputs = 2;
+  __device__ double operator()(double a, double b) const { return a + b; }
+};
+struct TriadOp {
+  static constexpr int kInputs = 2;
+  double alpha;
+  __device__ double operator()(double b, double c) const { return b + alpha * c; }
+};
 
-// ---- COPY ------------------------------------------------------------------
-template <int BS, int IT, typename V>
+template <typename Op>
+__device__ __forceinline__ double apply(const Op& f, double x, double y) { return f(x, y); }
+template <typename Op>
+__device__ __forceinline__ double2 apply(const Op& f, double2 x, double2 y) {
+  return make_double2(f(x.x, y.x), f(x.y, y.y));
+}
+
+// All loads of a tile are issued before its stores.  With 16-byte vectors an
+// odd n leaves one element, done by the first thread of the last CTA: a
+// second launch for it cost 2 us behind every call (n = 4099: 20 launches a
+// rep of the Stream, Basic and LCALS kernels instead of 16).
+template <int BS, int IT, typename V, typename Op>
 __global__ void __launch_bounds__(BS)
-copy_kernel(const V* __restrict__ a, V* __restrict__ c, int64_t units) {
-  TILE_LOOP(BS, IT, units) {
-    V r[IT];
-#pragma unroll
-    for (int u = 0; u < IT; ++u) {
-      int64_t j = t0 + u * BS + threadIdx.x;
-      if (j < units) r[u] = ldg(a + j);
-    }
-#pragma unroll
-    for (int u = 0; u < IT; ++u) {
-      int64_t j = t0 + u * BS + threadIdx.x;
-      if (j < units) c[j] = r[u];
-    }
-  }
-}
-
-// ---- MUL -------------------------------------------------------------------
-__device__ __forceinline__ double2 mul2(double s, double2 v) {
-  return make_double2(s * v.x, s * v.y);
-}
-__device__ __forceinline__ double mul2(double s, double v) { return s * v; }
-
-template <int BS, int IT, typename V>
-__global__ void __launch_bounds__(BS)
-mul_kernel(V* __restrict__ b, const V* __restrict__ c, double alpha,
-           int64_t units) {
-  TILE_LOOP(BS, IT, units) {
-    V r[IT];
-#pragma unroll
-    for (int u = 0; u < IT; ++u) {
-      int64_t j = t0 + u * BS + threadIdx.x;
-      if (j < units) r[u] = ldg(c + j);
-    }
-#pragma unroll
-    for (int u = 0; u < IT; ++u) {
-      int64_t j = t0 + u * BS + threadIdx.x;
-      if (j < units) b[j] = mul2(alpha, r[u]);
-    }
-  }
-}
-
-// ---- ADD -------------------------------------------------------------------
-__device__ __forceinline__ double2 add2(double2 x, double2 y) {
-  return make_double2(x.x + y.x, x.y + y.y);
-}
-__device__ __forceinline__ double add2(double x, double y) { return x + y; }
-
-template <int BS, int IT, typename V>
-__global__ void __launch_bounds__(BS)
-add_kernel(const V* __restrict__ a, const V* __restrict__ b,
-           V* __restrict__ c, int64_t units) {
+stream_kernel(const double* in1, const double* in2, double* out, Op f, int64_t n) {
+  constexpr int kVec = sizeof(V) / sizeof(double);
+  const int64_t first = begin() + threadIdx.x;
+  const V* a = reinterpret_cast<const V*>(in1);
+  const V* b = reinterpret_cast<const V*>(in2);
+  V* c = reinterpret_cast<V*>(out);
+  const int64_t units = n / kVec;
   TILE_LOOP(BS, IT, units) {
     V ra[IT], rb[IT];
 #pragma unroll
     for (int u = 0; u < IT; ++u) {
-      int64_t j = t0 + u * BS + threadIdx.x;
-      if (j < units) { ra[u] = ldg(a + j); rb[u] = ldg(b + j); }
+      const int64_t j = t0 + u * BS + first;
+      if (j < units) {
+        ra[u] = a[j];
+        if (Op::kInputs == 2) rb[u] = b[j];
+      }
     }
 #pragma unroll
     for (int u = 0; u < IT; ++u) {
-      int64_t j = t0 + u * BS + threadIdx.x;
-      if (j < units) c[j] = add2(ra[u], rb[u]);
+      const int64_t j = t0 + u * BS + first;
+      if (j < units) c[j] = apply(f, ra[u], Op::kInputs == 2 ? rb[u] : ra[u]);
     }
   }
-}
-
-// ---- TRIAD -----------------------------------------------------------------
-__device__ __forceinline__ double2 triad2(double2 b, double alpha, double2 c) {
-  return make_double2(b.x + alpha * c.x, b.y + alpha * c.y);
-}
-__device__ __forceinline__ double triad2(double b, double alpha, double c) {
-  return b + alpha * c;
-}
-
-template <int BS, int IT, typename V>
-__global__ void __launch_bounds__(BS)
-triad_kernel(V* __restrict__ a, const V* __restrict__ b,
-             const V* __restrict__ c, double alpha, int64_t units) {
-  TILE_LOOP(BS, IT, units) {
-    V rb[IT], rc[IT];
-#pragma unroll
-    for (int u = 0; u < IT; ++u) {
-      int64_t j = t0 + u * BS + threadIdx.x;
-      if (j < units) { rb[u] = ldg(b + j); rc[u] = ldg(c + j); }
-    }
-#pragma unroll
-    for (int u = 0; u < IT; ++u) {
-      int64_t j = t0 + u * BS + threadIdx.x;
-      if (j < units) a[j] = triad2(rb[u], alpha, rc[u]);
-    }
+  if (kVec == 2 && (n & 1) && blockIdx.x == gridDim.x - 1 && first == 0) {
+    const double x = in1[n - 1];
+    out[n - 1] = f(x, Op::kInputs == 2 ? in2[n - 1] : x);
   }
 }
 
@@ -125,11 +90,11 @@ triad_kernel(V* __restrict__ a, const V* __restrict__ b,
 // order; the last CTA combines the per-CTA partials in CTA order.
 template <int BS, int IT>
 __global__ void __launch_bounds__(BS)
-dot_kernel(const double* __restrict__ a, const double* __restrict__ b,
-           int64_t n, bool vec2, double dot_init, double* __restrict__ accum,
-           double* __restrict__ partials, unsigned int* __restrict__ counter) {
+dot_kernel(const double* a, const double* b, int64_t n, bool vec2, double dot_init,
+           double* accum, double* partials, unsigned int* counter) {
   __shared__ double smem[BS / 32];
   __shared__ bool last_flag;
+  const int64_t first = begin() + threadIdx.x;
   double s = 0.0;
   if (vec2) {
     const double2* a2 = reinterpret_cast<const double2*>(a);
@@ -139,27 +104,27 @@ dot_kernel(const double* __restrict__ a, const double* __restrict__ b,
       double2 ra[IT], rb[IT];
 #pragma unroll
       for (int u = 0; u < IT; ++u) {
-        int64_t j = t0 + u * BS + threadIdx.x;
-        if (j < units) { ra[u] = __ldg(a2 + j); rb[u] = __ldg(b2 + j); }
+        int64_t j = t0 + u * BS + first;
+        if (j < units) { ra[u] = a2[j]; rb[u] = b2[j]; }
       }
 #pragma unroll
       for (int u = 0; u < IT; ++u) {
-        int64_t j = t0 + u * BS + threadIdx.x;
+        int64_t j = t0 + u * BS + first;
         if (j < units) { s += ra[u].x * rb[u].x; s += ra[u].y * rb[u].y; }
       }
     }
-    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) s += a[n - 1] * b[n - 1];
+    if ((n & 1) && blockIdx.x == 0 && first == 0) s += a[n - 1] * b[n - 1];
   } else {
     TILE_LOOP(BS, IT, n) {
       double ra[IT], rb[IT];
 #pragma unroll
       for (int u = 0; u < IT; ++u) {
-        int64_t j = t0 + u * BS + threadIdx.x;
-        if (j < n) { ra[u] = __ldg(a + j); rb[u] = __ldg(b + j); }
+        int64_t j = t0 + u * BS + first;
+        if (j < n) { ra[u] = a[j]; rb[u] = b[j]; }
       }
 #pragma unroll
       for (int u = 0; u < IT; ++u) {
-        int64_t j = t0 + u * BS + threadIdx.x;
+        int64_t j = t0 + u * BS + first;
         if (j < n) s += ra[u] * rb[u];
       }
     }
@@ -178,30 +143,21 @@ dot_kernel(const double* __restrict__ a, const double* __restrict__ b,
   }
 }
 
-// Shared launcher for the four map kernels: vector path when every pointer
-// is 16-byte aligned, scalar path (and scalar tail) otherwise.
-template <typename LaunchVec, typename LaunchScalar>
-int launch_map(const char* name, int64_t n, const b200_tune* tune,
-               bool all_aligned, LaunchVec&& lv, LaunchScalar&& ls) {
-  Shape sh = resolve_1d(tune, 0, kBlock, kItems, 2);
-  if (!valid_block(sh.block)) return invalid("%s: bad block size %d", name, sh.block);
-  bool vec = all_aligned && sh.vec == 2 && n >= 2;
-  int launches = 0;
-  if (vec) {
-    int64_t units = n >> 1;
-    Shape s = resolve_1d(tune, units, kBlock, kItems, 2);
-    lv(s, units);
-    ++launches;
-    if (n & 1) {
-      ls(Shape{32, 1, 1, 1}, n - 1, int64_t{1});
-      ++launches;
-    }
-  } else {
-    Shape s = resolve_1d(tune, n, kBlock, kItems, 1);
-    ls(s, int64_t{0}, n);
-    ++launches;
-  }
-  return after_launch(name, launches);
+// Shared launcher: the vector path when every pointer is 16-byte aligned, the
+// scalar one otherwise.  A short array takes fewer items per thread (spread).
+template <typename Op>
+int launch_stream(const char* name, const double* in1, const double* in2, double* out, Op f,
+                  int64_t n, const b200_tune* tune, cudaStream_t st) {
+  if (n == 0) return B200_OK;
+  const bool vec = aligned16(in1) && aligned16(in2) && aligned16(out) && n >= 2 &&
+                   !(tune && tune->vec && tune->vec != 2);
+  const int64_t units = vec ? n >> 1 : n;
+  const Shape s = resolve_1d(tune, units, kBlock, spread(units, kBlock, kItems), vec ? 2 : 1);
+  if (!valid_block(s.block)) return invalid("%s: bad block size %d", name, s.block);
+  B200_DISPATCH_BLOCK(s.block, BS, B200_DISPATCH_ITEMS(s.items, IT,
+    if (vec) launch(stream_kernel<BS, IT, double2, Op>, s.grid, BS, 0, st, in1, in2, out, f, n);
+    else launch(stream_kernel<BS, IT, double, Op>, s.grid, BS, 0, st, in1, in2, out, f, n)));
+  return after_launch(name);
 }
 
 }  // namespace
@@ -211,63 +167,20 @@ extern "C" {
 int b200_stream_copy(const double* a, double* c, int64_t n,
                      const b200_tune* tune, b200_stream_t stream) {
   if (n < 0 || (n > 0 && (!a || !c))) return invalid("b200_stream_copy: bad args");
-  if (n == 0) return B200_OK;
-  cudaStream_t st = as_stream(stream);
-  return launch_map(
-      "b200_stream_copy", n, tune, aligned16(a) && aligned16(c),
-      [&](Shape s, int64_t units) {
-        B200_DISPATCH_BLOCK(s.block, BS, B200_DISPATCH_ITEMS(s.items, IT,
-          copy_kernel<BS, IT, double2><<<s.grid, BS, 0, st>>>(
-              reinterpret_cast<const double2*>(a),
-              reinterpret_cast<double2*>(c), units)));
-      },
-      [&](Shape s, int64_t off, int64_t cnt) {
-        B200_DISPATCH_BLOCK(s.block, BS, B200_DISPATCH_ITEMS(s.items, IT,
-          copy_kernel<BS, IT, double><<<s.grid, BS, 0, st>>>(a + off, c + off,
-                                                             cnt)));
-      });
+  return launch_stream("b200_stream_copy", a, a, c, CopyOp{}, n, tune, as_stream(stream));
 }
 
 int b200_stream_mul(double* b, const double* c, double alpha, int64_t n,
                     const b200_tune* tune, b200_stream_t stream) {
   if (n < 0 || (n > 0 && (!b || !c))) return invalid("b200_stream_mul: bad args");
-  if (n == 0) return B200_OK;
-  cudaStream_t st = as_stream(stream);
-  return launch_map(
-      "b200_stream_mul", n, tune, aligned16(b) && aligned16(c),
-      [&](Shape s, int64_t units) {
-        B200_DISPATCH_BLOCK(s.block, BS, B200_DISPATCH_ITEMS(s.items, IT,
-          mul_kernel<BS, IT, double2><<<s.grid, BS, 0, st>>>(
-              reinterpret_cast<double2*>(b),
-              reinterpret_cast<const double2*>(c), alpha, units)));
-      },
-      [&](Shape s, int64_t off, int64_t cnt) {
-        B200_DISPATCH_BLOCK(s.block, BS, B200_DISPATCH_ITEMS(s.items, IT,
-          mul_kernel<BS, IT, double><<<s.grid, BS, 0, st>>>(b + off, c + off,
-                                                            alpha, cnt)));
-      });
+  return launch_stream("b200_stream_mul", c, c, b, MulOp{alpha}, n, tune, as_stream(stream));
 }
 
 int b200_stream_add(const double* a, const double* b, double* c, int64_t n,
                     const b200_tune* tune, b200_stream_t stream) {
   if (n < 0 || (n > 0 && (!a || !b || !c)))
     return invalid("b200_stream_add: bad args");
-  if (n == 0) return B200_OK;
-  cudaStream_t st = as_stream(stream);
-  return launch_map(
-      "b200_stream_add", n, tune, aligned16(a) && aligned16(b) && aligned16(c),
-      [&](Shape s, int64_t units) {
-        B200_DISPATCH_BLOCK(s.block, BS, B200_DISPATCH_ITEMS(s.items, IT,
-          add_kernel<BS, IT, double2><<<s.grid, BS, 0, st>>>(
-              reinterpret_cast<const double2*>(a),
-              reinterpret_cast<const double2*>(b),
-              reinterpret_cast<double2*>(c), units)));
-      },
-      [&](Shape s, int64_t off, int64_t cnt) {
-        B200_DISPATCH_BLOCK(s.block, BS, B200_DISPATCH_ITEMS(s.items, IT,
-          add_kernel<BS, IT, double><<<s.grid, BS, 0, st>>>(
-              a + off, b + off, c + off, cnt)));
-      });
+  return launch_stream("b200_stream_add", a, b, c, AddOp{}, n, tune, as_stream(stream));
 }
 
 int b200_stream_triad(double* a, const double* b, const double* c,
@@ -275,23 +188,8 @@ int b200_stream_triad(double* a, const double* b, const double* c,
                       b200_stream_t stream) {
   if (n < 0 || (n > 0 && (!a || !b || !c)))
     return invalid("b200_stream_triad: bad args");
-  if (n == 0) return B200_OK;
-  cudaStream_t st = as_stream(stream);
-  return launch_map(
-      "b200_stream_triad", n, tune,
-      aligned16(a) && aligned16(b) && aligned16(c),
-      [&](Shape s, int64_t units) {
-        B200_DISPATCH_BLOCK(s.block, BS, B200_DISPATCH_ITEMS(s.items, IT,
-          triad_kernel<BS, IT, double2><<<s.grid, BS, 0, st>>>(
-              reinterpret_cast<double2*>(a),
-              reinterpret_cast<const double2*>(b),
-              reinterpret_cast<const double2*>(c), alpha, units)));
-      },
-      [&](Shape s, int64_t off, int64_t cnt) {
-        B200_DISPATCH_BLOCK(s.block, BS, B200_DISPATCH_ITEMS(s.items, IT,
-          triad_kernel<BS, IT, double><<<s.grid, BS, 0, st>>>(
-              a + off, b + off, c + off, alpha, cnt)));
-      });
+  return launch_stream("b200_stream_triad", b, c, a, TriadOp{alpha}, n, tune,
+                       as_stream(stream));
 }
 
 size_t b200_reduce_workspace_bytes(int64_t n, const b200_tune* tune) {
@@ -322,8 +220,8 @@ int b200_stream_dot(const double* a, const double* b, int64_t n,
   double* partials = reinterpret_cast<double*>(static_cast<char*>(workspace) + 256);
   cudaStream_t st = as_stream(stream);
   B200_DISPATCH_BLOCK(block, BS, B200_DISPATCH_ITEMS(items, IT,
-    dot_kernel<BS, IT><<<grid, BS, 0, st>>>(a, b, n, vec, dot_init, dot_accum,
-                                            partials, counter)));
+    launch(dot_kernel<BS, IT>, grid, BS, 0, st, a, b, n, vec, dot_init, dot_accum, partials,
+           counter)));
   return after_launch("b200_stream_dot");
 }
 
