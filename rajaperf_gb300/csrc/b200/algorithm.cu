@@ -1,19 +1,20 @@
 // Algorithm group: SCAN (exclusive prefix sum, FP64 and int64) and REDUCE_SUM.
 //
-// SCAN is a single-pass decoupled-lookback scan: every CTA takes the next
-// tile id from a counter (so a CTA only ever waits on tiles already owned by
-// running CTAs).  A dedicated lookback warp starts walking its predecessors'
-// aggregates / inclusive prefixes at once, while eight loader warps stage
-// the tile in shared memory, reduce it and publish its aggregate; the
-// lookback warp then publishes the tile's inclusive prefix and the loaders
-// write the tile out.  Flags carry a launch epoch, so the workspace never
-// needs re-zeroing between calls (and the call can be captured in a CUDA
-// graph): the CTA that draws the launch's last tile id resets the tile
-// counter and advances the epoch.  Every wait is bounded; a wait that gives up sets the error word of
-// the workspace header (byte offset 16) and the call's results are invalid.
+// SCAN is a single-pass scan: every CTA takes the next tile id from a counter
+// (so a CTA only ever waits on tiles already owned by running CTAs).  Three
+// kernels: one CTA per tile with a lookback warp (scan_kernel), and two
+// persistent ones on a ring of shared-memory stages, for int64 with lookback
+// warps (pipe::scan_pipelined), for FP64 with one scanner warp that gives all
+// tiles their prefixes (pipe64::scan_pipelined_f64).  Flags carry a launch
+// epoch, so the workspace never needs re-zeroing between calls (and the call
+// can be captured in a CUDA graph): the CTA that draws the launch's last tile
+// id resets the tile counter and advances the epoch.  Every wait is bounded; a
+// wait that gives up sets the error word of the workspace header (byte offset
+// 16) and the call's results are invalid.
 #include "b200_internal.cuh"
 #include "b200_fma_form.cuh"
 #include "b200_async.cuh"
+#include "b200_f64emu.cuh"
 #include "b200_launch.cuh"
 #include "b200_lookback.cuh"
 #include "b200_pipeline.cuh"
@@ -208,7 +209,7 @@ struct Smem {
 
 template <typename T>
 constexpr size_t smem_bytes() { return sizeof(Smem<T>) + 128; }
-static_assert(sizeof(Smem<double>) + 128 <= 232448, "shared memory budget");
+static_assert(sizeof(Smem<long long>) + 128 <= 232448, "shared memory budget");
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -355,6 +356,451 @@ scan_pipelined(const T* __restrict__ x, T* __restrict__ y, int64_t n, T init,
 
 }  // namespace pipe
 
+// ---- pipelined persistent SCAN, FP64 ----------------------------------------
+// The ring again, arranged around the FP64 pipe, which bounds an FP64 scan: at
+// 2 thread instructions per clock and SM (595 G/s), the tile kernel's three
+// adds per item (run total, prefix in the tile, plus the tile's prefix) take
+// 0.40 ms at 2^26 items, the memory traffic 0.16 ms.  Here an item costs one
+// or two:
+//  * four aggregator warps total the runs on the integer pipes.  Items of one
+//    sign add exactly as integers in units of 2^-56 of the largest one's
+//    binade (what an item has below that is cut: less than 2^-56 of the run's
+//    total), and the total is rounded once, where a chain of FP64 adds rounds
+//    34 times.  A run of both signs, whose total may cancel, or with an
+//    infinity, a NaN or nothing above 2^-960, is totalled with FP64 adds.
+//  * two groups of four compute warps take alternate tiles, a thread a run of
+//    34 consecutive items.  Where the tile's exclusive prefix has the run's
+//    sign and is at least 2^16 times its largest item's binade, the prefix in
+//    the tile is summed as an integer too (units of 2^-49 of that binade 2^e,
+//    rounded to 2^-38 of it: at most an eighth of the result's last place), set
+//    as the low bits of a double D = 2^(e+14) + prefix, and the result is
+//    (exclusive - 2^(e+14)) + D: the difference is exact, so one FP64 add and
+//    one rounding per item.  Elsewhere (the first tiles, mixed signs) a chain
+//    of FP64 adds gives the prefix in the tile and one more the result.
+// 17 pairs per run: an odd stride of 16-byte accesses is free of bank
+// conflicts with every run in order.  No barrier joins the warps of a role;
+// each arrives on the stage's mbarrier by itself.
+namespace pipe64 {
+
+using ring::kEnd;
+constexpr int kAggWarps = 4;
+constexpr int kGroups = 2;                    // compute groups, alternate tiles
+constexpr int kGroupWarps = kAggWarps;        // a run has the same lane in both roles
+constexpr int kFirstAgg = 2;                  // after the producer and the prefix warp
+constexpr int kFirstCompute = kFirstAgg + kAggWarps;
+constexpr int kStoreWarp = kFirstCompute + kGroups * kGroupWarps;
+constexpr int kThreads = 32 * (kStoreWarp + 1);
+constexpr int kRuns = 32 * kAggWarps;         // 128 runs per tile
+constexpr int kPairs = 17;
+constexpr int kTile = kRuns * kPairs * 2;     // 4352 items
+constexpr int kStages = 6;
+static_assert(kAggWarps == 4, "warp totals are summed as four");
+static_assert(kTile >= kScanTileMin, "the workspace has a descriptor per kScanTileMin items");
+
+struct Smem {
+  ring::Ring<double, double, kTile, kStages> r;
+  double before[kStages][kRuns];           // total of the warp's runs before this one
+  double warp_total[kStages][kAggWarps];
+  unsigned int top[kStages][kRuns];        // sign and exponent of the run's largest item, or 0
+  unsigned int arrived[kStages];           // aggregator warps done with the stage
+  uint64_t ready[kStages];                 // compute -> store warp: the stage holds results
+  unsigned long long ticket;               // the CTA's first
+};
+constexpr size_t kSmemBytes = sizeof(Smem) + 128;
+static_assert(kSmemBytes <= 232448, "shared memory budget");
+
+// v >> s for any s (0 from 64 on)
+__device__ __forceinline__ uint64_t shr(uint64_t v, uint32_t s) {
+  uint64_t r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
+  return r;
+}
+
+// The item's significand in units of 2^-UNIT of `top`'s binade; `top` is the
+// sign and exponent field of an item of the same sign that is no smaller, at
+// least 64, so that a zero's or subnormal's hidden bit is shifted out.
+template <int UNIT>
+__device__ __forceinline__ uint64_t fixed(uint64_t item, uint32_t top) {
+  const uint64_t m = (item & f64emu::kFrac) | f64emu::kHidden;
+  const uint32_t d = top - static_cast<uint32_t>(item >> 52);
+  if constexpr (UNIT >= 52) return shr(m << (UNIT - 52), d);
+  return shr(m, d + (52u - UNIT));
+}
+
+// v * 2^(unit - 1023), rounded to nearest even, on the integer pipes; `unit`
+// carries the sign above its 11 bits, and the result is a normal number.
+__device__ __forceinline__ double to_double(uint64_t v, uint32_t unit) {
+  if (v == 0u) return 0.0;
+  const uint32_t lz = static_cast<uint32_t>(__clzll(static_cast<long long>(v)));
+  const uint64_t w = v << lz, m = w >> 11;
+  const uint32_t up = ((static_cast<uint32_t>(w) & 0x7ffu) + 0x3ffu +
+                       (static_cast<uint32_t>(m) & 1u)) >> 11;
+  return f64emu::from_bits((static_cast<uint64_t>(unit + 62u - lz) << 52) + m + up);
+}
+
+// Prefix sums over a warp that stay off the FP64 pipe, where the aggregates'
+// dependent adds would queue behind the compute warps': one non-negative
+// integer per lane in units of 2^(top - 1023 - UNIT), all lanes' signs equal,
+// is brought to the warp's largest `top` (`all`) and, where 32 of them could
+// overflow, to a coarser unit.
+struct WarpFixed {
+  uint64_t v;
+  uint32_t unit;
+};
+template <int UNIT>
+__device__ __forceinline__ WarpFixed warp_align(uint64_t v, uint32_t top, uint32_t all) {
+  v = shr(v, all - top);
+  const uint32_t big = __reduce_max_sync(0xffffffffu, static_cast<uint32_t>(v >> 32));
+  const int lz = __clz(static_cast<int>(big));
+  const uint32_t s = lz < 5 ? 5u - lz : 0u;
+  return {(v + ((1ull << s) >> 1)) >> s, all - UNIT + s};
+}
+
+// The scanner: one warp, in a CTA that takes no tiles, turns the tiles'
+// aggregates, as they are published, into exclusive prefixes, in tile order.
+// Each tile's prefix warp then polls one descriptor, where a lookback re-reads
+// hundreds: at 2^26 items lookback warps in every CTA left the kernel at
+// 238-275 us (2 to 5 warps, 128 to 256 predecessors a round), the scanner at
+// 203 us (2, 4, 8 tiles per lane: 267, 203, 227 us; no prefixes at all: 173
+// us; the copy alone: 157 us).  A round takes the published tiles
+// from p on, up to kPerLane per lane.  The running prefix is kept in two parts
+// (Dekker's two-sum, larger operand first, compared as integers), so that its
+// roundings do not add up over the rounds.
+constexpr int kPerLane = 4;
+
+__device__ void scan_aggregates(TileDesc* descs, unsigned int tiles, double init,
+                                unsigned long long epoch, ScanHeader* hdr, uint64_t limit_ns) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long AGG = epoch * 4 + 1, INC = epoch * 4 + 2;
+  double hi = init, lo = 0.0;
+  uint64_t t0 = 0;  // time of the first empty round since the last full one
+  for (unsigned int p = 0; p < tiles;) {
+    double v[kPerLane];
+    unsigned int have = 0;  // the lane's published tiles before its first other one
+    {
+      unsigned long long f[kPerLane], bits[kPerLane];
+      const unsigned int t = p + lane * kPerLane;
+#pragma unroll
+      for (int j = 0; j < kPerLane; ++j) {
+        f[j] = bits[j] = 0ull;
+        if (t + j < tiles) desc_load(descs + t + j, f[j], bits[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < kPerLane; ++j) {
+        if (have == j && f[j] == AGG) ++have;
+        v[j] = have > j ? from_bits<double>(bits[j]) : 0.0;
+      }
+    }
+    const unsigned int part = __ballot_sync(0xffffffffu, have < kPerLane);
+    const int last = part ? __ffs(part) - 1 : 31;  // the last lane that counts
+    if (lane > last) have = 0;
+    const unsigned int found = last * kPerLane + __shfl_sync(0xffffffffu, have, last);
+    if (found == 0) {
+      uint64_t now = 0;
+      if (lane == 0) now = globaltimer();
+      now = __shfl_sync(0xffffffffu, now, 0);
+      if (t0 == 0) t0 = now;
+      if (now - t0 > limit_ns) {
+        if (lane == 0) atomicExch(&hdr->error, 1u);
+        return;
+      }
+      continue;
+    }
+    t0 = 0;
+    if (lane > last) {
+#pragma unroll
+      for (int j = 0; j < kPerLane; ++j) v[j] = 0.0;
+    }
+    double before[kPerLane];
+    double sum = 0.0;
+#pragma unroll
+    for (int j = 0; j < kPerLane; ++j) {
+      before[j] = sum;
+      sum += v[j];
+    }
+    const double inc = warp_inclusive_scan(sum);
+    double left = __shfl_up_sync(0xffffffffu, inc, 1);
+    left = lane == 0 ? lo : left + lo;
+#pragma unroll
+    for (int j = 0; j < kPerLane; ++j)
+      if (j < have)
+        desc_store(descs + p + lane * kPerLane + j, INC, to_bits<double>(hi + (left + before[j])));
+    const double all = __shfl_sync(0xffffffffu, inc, 31);
+    const bool first = (f64emu::bits_opaque(hi) << 1) >= (f64emu::bits_opaque(all) << 1);
+    const double a = first ? hi : all, b = first ? all : hi;
+    hi = a + b;
+    const double err = b - (hi - a);
+    lo += fabs(err) < INFINITY ? err : 0.0;
+    p += found;
+  }
+}
+
+// The prefix warp: takes each tile's exclusive prefix from the scanner.
+__device__ void fetch_prefixes(Smem& sm, const TileDesc* descs, double init, ScanHeader* hdr) {
+  auto& r = sm.r;
+  const int lane = threadIdx.x & 31;
+  for (int k = 0;; ++k) {
+    const int s = k % kStages;
+    if (!ring::wait(r, &r.drawn[s], (k / kStages) & 1, hdr)) return;
+    const unsigned int tile = r.ticket[s];
+    if (tile == kEnd) return;
+    if (lane == 0) {
+      const unsigned long long INC = r.epoch * 4 + 2;
+      double excl = init;
+      bool ok = true;
+      if (tile > 0) {
+        unsigned long long f, bits;
+        desc_load(descs + tile, f, bits);
+        if (f != INC) {
+          const uint64_t t0 = globaltimer();
+          while (ok && f != INC) {
+            desc_load(descs + tile, f, bits);
+            ok = globaltimer() - t0 <= r.limit_ns;
+          }
+        }
+        excl = from_bits<double>(bits);
+      }
+      if (ok) {
+        r.excl[s] = excl;
+        mbar_arrive(&r.prefix[s]);
+      } else {
+        atomicExch(&hdr->error, 1u);
+        *reinterpret_cast<volatile int*>(&r.abort) = 1;
+      }
+    }
+    __syncwarp();
+    if (*reinterpret_cast<volatile int*>(&r.abort)) return;
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+scan_pipelined_f64(const double* x, double* y, int64_t n, double init, unsigned int tiles,
+                   ScanHeader* hdr, TileDesc* descs, uint64_t limit_ns, int zero) {
+  extern __shared__ unsigned char s_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>(
+      (reinterpret_cast<uintptr_t>(s_raw) + 127) & ~static_cast<uintptr_t>(127));
+  auto& r = sm.r;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+  if (tid == 0) {
+    ring::init(r, limit_ns);
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&sm.ready[s], kGroupWarps);
+      sm.arrived[s] = 0u;
+    }
+    mbar_init_fence();
+  }
+  const unsigned int z = begin();
+  x += z;
+  hdr += z;
+  descs += z;
+  if (tid == 0) {
+    const unsigned long long draws = static_cast<unsigned long long>(tiles) + gridDim.x;
+    const unsigned long long t = atomicAdd(&hdr->ticket, 1ull);
+    if (static_cast<unsigned int>(t) == draws - 1)
+      atomicAdd(&hdr->ticket, (1ull << 32) - draws);
+    sm.ticket = t;
+  }
+  __syncthreads();
+  // the CTA with the first ticket scans the aggregates of all the others (a
+  // single tile needs no scanner)
+  const unsigned int bias = tiles > 1u ? 1u : 0u;
+  if (static_cast<unsigned int>(sm.ticket) < bias) {
+    if (warp == 0) scan_aggregates(descs, tiles, init, sm.ticket >> 32, hdr, limit_ns);
+    return;
+  }
+
+  if (warp == 0) {
+    ring::produce(r, x, n, tiles, hdr, kGroups, &sm.ticket, bias);
+  } else if (warp < kFirstAgg) {
+    fetch_prefixes(sm, descs, init, hdr);
+  } else if (warp < kFirstCompute) {
+    // ---- aggregators ----
+    const int aw = warp - kFirstAgg, run = aw * 32 + lane;
+    for (int k = 0;; ++k) {
+      const int s = k % kStages;
+      if (!ring::wait(r, &r.full[s], (k / kStages) & 1, hdr)) break;
+      const unsigned int tile = r.ticket[s];
+      if (tile == kEnd) break;
+      const ulonglong2* tv = reinterpret_cast<const ulonglong2*>(r.tile[s]) + run * kPairs;
+      ulonglong2 v[kPairs];
+      uint32_t top = 0u, differ = 0u;  // largest high word; its sign bit: signs differ
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) v[q] = tv[q];
+      const uint32_t first = static_cast<uint32_t>(v[0].x >> 32);
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) {
+        const uint32_t a = static_cast<uint32_t>(v[q].x >> 32);
+        const uint32_t b = static_cast<uint32_t>(v[q].y >> 32);
+        top = max(top, max(a, b));
+        differ |= (a ^ first) | (b ^ first);
+      }
+      top >>= 20;
+      const uint32_t e = top & 0x7ffu;
+      double before, inc;  // totals of the warp's runs before this one, and up to it
+      const bool one_sign = (differ >> 31) == 0u && e - 64u < 2032u - 64u;
+      uint64_t acc = 0;  // at most 34 * (2^57 - 1)
+      if (one_sign) {
+#pragma unroll
+        for (int q = 0; q < kPairs; ++q) acc += fixed<56>(v[q].x, top) + fixed<56>(v[q].y, top);
+      } else {
+        top = 0u;
+      }
+      const uint32_t most = __reduce_max_sync(0xffffffffu, top);
+      // runs of one size and sign: no run loses bits to a later one
+      if (__all_sync(0xffffffffu, one_sign && most - top < 4u)) {
+        const WarpFixed f = warp_align<56>(acc, top, most);
+        const uint64_t up_to = warp_inclusive_scan(f.v);
+        inc = to_double(up_to, f.unit);
+        before = to_double(up_to - f.v, f.unit);
+      } else {
+        double total;
+        if (one_sign) {
+          total = to_double(acc, top - 56u);
+        } else {
+          total = 0.0;
+#pragma unroll
+          for (int q = 0; q < kPairs; ++q) {
+            total += f64emu::from_bits(v[q].x);
+            total += f64emu::from_bits(v[q].y);
+          }
+        }
+        inc = warp_inclusive_scan(total);
+        before = __shfl_up_sync(0xffffffffu, inc, 1);
+        if (lane == 0) before = 0.0;
+      }
+      sm.before[s][run] = before;
+      sm.top[s][run] = top;
+      if (lane == 31) sm.warp_total[s][aw] = inc;
+      __syncwarp();
+      if (lane == 0) {
+        __threadfence_block();
+        if (atomicAdd(&sm.arrived[s], 1u) == kAggWarps - 1u) {  // the last of the four
+          __threadfence_block();
+          sm.arrived[s] = 0u;
+          volatile double* wt = sm.warp_total[s];
+          const double w0 = wt[0], w1 = wt[1], w2 = wt[2], w3 = wt[3], w01 = w0 + w1;
+          desc_store(descs + tile, r.epoch * 4 + 1, to_bits<double>(w01 + (w2 + w3)));
+          wt[0] = 0.0;  // now the totals of the warps before
+          wt[1] = w0;
+          wt[2] = w01;
+          wt[3] = w01 + w2;
+          mbar_arrive(&r.summed[s]);
+        }
+      }
+      __syncwarp();
+    }
+  } else if (warp < kStoreWarp) {
+    // ---- compute ----
+    const int group = (warp - kFirstCompute) / kGroupWarps;
+    const int cw = (warp - kFirstCompute) % kGroupWarps, run = cw * 32 + lane;
+    const fform::Regs rg = fform::regs(zero);
+    for (int k = group;; k += kGroups) {
+      const int s = k % kStages;
+      const uint32_t par = (k / kStages) & 1;
+      if (!ring::wait(r, &r.drawn[s], par, hdr)) break;
+      const unsigned int tile = r.ticket[s];
+      if (tile == kEnd) break;
+      if (!ring::wait(r, &r.full[s], par, hdr)) break;
+      if (!ring::wait(r, &r.summed[s], par, hdr)) break;
+      double2* tv = reinterpret_cast<double2*>(r.tile[s]) + run * kPairs;
+      double2 v[kPairs];
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) v[q] = tv[q];
+      double off = sm.before[s][run] + sm.warp_total[s][cw];  // the tile's total before this run
+      // signs and exponents: of the run's largest item, of off
+      const uint32_t top = sm.top[s][run], e = top & 0x7ffu;
+      const uint64_t ob = f64emu::bits(off);
+      const uint32_t oe = static_cast<uint32_t>(ob >> 52);
+      const uint64_t head = static_cast<uint64_t>(top + 14u) << 52;  // 2^(e+14)
+      auto chain = [&] {
+        double o = off;
+#pragma unroll
+        for (int q = 0; q < kPairs; ++q) {
+          const double a = v[q].x, b = v[q].y;
+          v[q].x = o;
+          o = fform::add(a, o, rg);
+          v[q].y = o;
+          o = fform::add(b, o, rg);
+        }
+      };
+      // off is below 2^(e+13), the run's total below 2^(e+7)
+      bool whole = top != 0u && (ob == 0u || oe - (top & 0x800u) < e + 13u);
+      if (whole) {
+        uint64_t acc = 1024u;
+        if (ob != 0u)
+          acc += shr(((ob & f64emu::kFrac) | f64emu::kHidden) << 10, e + 13u - (oe & 0x7ffu));
+#pragma unroll
+        for (int q = 0; q < kPairs; ++q) {
+          const uint64_t a = f64emu::bits(v[q].x), b = f64emu::bits(v[q].y);
+          v[q].x = f64emu::from_bits(head | (acc >> 11));
+          acc += fixed<49>(a, top);
+          v[q].y = f64emu::from_bits(head | (acc >> 11));
+          acc += fixed<49>(b, top);
+        }
+      } else {
+        chain();
+      }
+      if (!ring::wait(r, &r.prefix[s], par, hdr)) break;
+      double rest = r.excl[s];
+      const uint32_t xe = static_cast<uint32_t>(f64emu::bits(rest) >> 52);
+      if (whole) {
+        // up to xe = e + 66, 2^(e+14) is a multiple of the prefix's last place
+        if (xe - (top + 16u) <= 50u && ((xe ^ top) & 0x800u) == 0u) {
+          rest -= f64emu::from_bits(head);
+        } else {
+#pragma unroll
+          for (int q = 0; q < kPairs; ++q) v[q] = tv[q];
+          chain();
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) {
+        v[q].x = fform::add(v[q].x, rest, rg);
+        v[q].y = fform::add(v[q].y, rest, rg);
+      }
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) tv[q] = v[q];
+      fence_proxy_async_smem();
+      __syncwarp();
+      const int64_t first = static_cast<int64_t>(tile) * kTile;
+      if (first + kTile > n) {  // the ragged last tile: plain stores of the warp's own items
+        constexpr int kOwn = 32 * 2 * kPairs;
+        for (int i = cw * kOwn + lane; i < (cw + 1) * kOwn; i += 32)
+          if (first + i < n) y[first + i] = r.tile[s][i];
+        __syncwarp();
+      }
+      if (lane == 0) mbar_arrive(&sm.ready[s]);
+    }
+  } else {
+    // ---- store: one bulk store per finished tile, then the stage is free ----
+    for (int k = 0;; ++k) {
+      const int s = k % kStages;
+      const uint32_t par = (k / kStages) & 1;
+      if (!ring::wait(r, &r.drawn[s], par, hdr)) break;
+      const unsigned int tile = r.ticket[s];
+      if (tile == kEnd) break;
+      if (!ring::wait(r, &sm.ready[s], par, hdr)) break;
+      const int64_t first = static_cast<int64_t>(tile) * kTile;
+      if (lane == 0) {
+        if (first + kTile <= n) {
+          bulk_store(y + first, r.tile[s], kTile * sizeof(double));
+          bulk_commit();
+          bulk_wait_read<0>();
+        }
+        mbar_arrive(&r.empty[s]);
+      }
+      __syncwarp();
+    }
+    if (lane == 0) bulk_wait_all();
+  }
+
+  __syncthreads();
+  if (tid == 0) ring::drain(r);
+}
+
+}  // namespace pipe64
+
 // The workspace is sized for the smallest tile, so it serves every tile size.
 int64_t scan_tiles_max(int64_t n) { return ceil_div(n > 0 ? n : 1, kScanTileMin); }
 
@@ -374,18 +820,31 @@ int launch_scan_it(const T* x, T* y, int64_t n, T init, char* w, uint64_t limit_
   return B200_OK;
 }
 
-template <typename T>
-int launch_scan_pipelined(const T* x, T* y, int64_t n, T init, char* w, uint64_t limit_ns,
-                          cudaStream_t st) {
-  constexpr size_t kSmem = pipe::smem_bytes<T>();
-  const int rc = allow_dynamic_smem(reinterpret_cast<const void*>(pipe::scan_pipelined<T>),
-                                    kSmem, "scan");
+int launch_scan_pipelined(const long long* x, long long* y, int64_t n, long long init, char* w,
+                          uint64_t limit_ns, cudaStream_t st) {
+  constexpr size_t kSmem = pipe::smem_bytes<long long>();
+  const int rc = allow_dynamic_smem(
+      reinterpret_cast<const void*>(pipe::scan_pipelined<long long>), kSmem, "scan");
   if (rc != B200_OK) return rc;
   const int64_t tiles = ceil_div(n, pipe::kTile);
   const int grid = static_cast<int>(std::min<int64_t>(tiles, device_info().sm_count));
-  pipe::scan_pipelined<T><<<grid, pipe::kThreads, kSmem, st>>>(
+  pipe::scan_pipelined<long long><<<grid, pipe::kThreads, kSmem, st>>>(
       x, y, n, init, static_cast<unsigned int>(tiles), reinterpret_cast<ScanHeader*>(w),
       reinterpret_cast<TileDesc*>(w + 256), limit_ns);
+  return B200_OK;
+}
+
+int launch_scan_pipelined(const double* x, double* y, int64_t n, double init, char* w,
+                          uint64_t limit_ns, cudaStream_t st) {
+  const int rc = allow_dynamic_smem(reinterpret_cast<const void*>(pipe64::scan_pipelined_f64),
+                                    pipe64::kSmemBytes, "scan");
+  if (rc != B200_OK) return rc;
+  const int64_t tiles = ceil_div(n, pipe64::kTile);
+  const int grid =
+      static_cast<int>(std::min<int64_t>(tiles > 1 ? tiles + 1 : 1, device_info().sm_count));
+  launch(pipe64::scan_pipelined_f64, grid, pipe64::kThreads, pipe64::kSmemBytes, st, x, y, n,
+         init, static_cast<unsigned int>(tiles), reinterpret_cast<ScanHeader*>(w),
+         reinterpret_cast<TileDesc*>(w + 256), limit_ns, 0);
   return B200_OK;
 }
 
@@ -400,7 +859,11 @@ int launch_scan(const char* name, const T* x, T* y, int64_t n, T init, void* ws,
   if (algo < 0 || algo > 2) return invalid("%s: algo %d (0, 1 or 2)", name, algo);
   if (tune && tune->block_size && tune->block_size != kScanBlock)
     return invalid("%s: block size %d (only %d)", name, tune->block_size, kScanBlock);
-  const int items = (tune && tune->items) ? tune->items : kScanItemsDefault;
+  // up to one tile of 4096 items per SM the tile kernel takes those (500001
+  // items of FP64: 9.9 us against 12.4 with 8192)
+  const bool one_wave = n <= static_cast<int64_t>(device_info().sm_count) * kScanTileMin;
+  const int items = (tune && tune->items) ? tune->items
+                                          : (one_wave ? kScanItemsMin : kScanItemsDefault);
   if (items != 16 && items != 32) return invalid("%s: items %d (16 or 32)", name, items);
   size_t need = 256 + static_cast<size_t>(slots) * sizeof(TileDesc);
   if (ws && !aligned16(ws)) return invalid("%s: workspace not 16-byte aligned", name);
@@ -412,11 +875,12 @@ int launch_scan(const char* name, const T* x, T* y, int64_t n, T init, void* ws,
   const bool vec = aligned16(x) && aligned16(y) && !(tune && tune->vec == 1);
   const uint64_t lim = wait_limit_ns(tune, kDefaultWaitNs);
   int rc;
-  // the ring's aggregator warp sums a tile on one sub-partition's FP64 unit
-  // (FP64-bound at 4 us per tile), so FP64 takes the tile kernel by default
-  const bool ring = vec && (algo == 2 || (algo == 0 && std::is_same<T, long long>::value));
+  // FP64 takes the tile kernel for as long as it is one wave (65536 items: 8.4
+  // us, the ring 11 us; 700001: 13.4 and 11.1 us; 2^26: 467 and 203 us)
+  const bool ring =
+      vec && (algo == 2 || (algo == 0 && (std::is_same<T, long long>::value || !one_wave)));
   if (ring)
-    rc = launch_scan_pipelined<T>(x, y, n, init, w, lim, st);
+    rc = launch_scan_pipelined(x, y, n, init, w, lim, st);
   else
     rc = (items == 16) ? (vec ? launch_scan_it<T, 16, true>(x, y, n, init, w, lim, st)
                               : launch_scan_it<T, 16, false>(x, y, n, init, w, lim, st))

@@ -1,6 +1,6 @@
-// The stage ring of SCAN's persistent single-pass lookback kernel: one CTA
-// per SM streams tiles of 4096 items of a 1-D array through seven
-// shared-memory stages.  This header holds the ring's layout and bounded
+// The stage ring of SCAN's persistent single-pass lookback kernels: one CTA
+// per SM streams tiles of a 1-D array (4096 items by default) through its
+// shared-memory stages (seven by default).  This header holds the ring's layout and bounded
 // waits, the producer warp (draws tile ids, issues one bulk copy per tile)
 // and the lookback warps (walk back to the nearest inclusive prefix, publish
 // the tile's own); the kernel adds an aggregator warp (publishes a tile's
@@ -35,15 +35,18 @@
 namespace b200 {
 namespace ring {
 
-constexpr int kTile = 4096;                  // items per tile
+constexpr int kTile = 4096;                  // items per tile, unless a kernel says otherwise
 constexpr int kStages = 7;
 constexpr int kLookbackWarps = 2;
 constexpr int kLookbackLanes = 8;            // 256 predecessors per lookback round
 constexpr unsigned int kEnd = 0xffffffffu;   // end marker in ticket[]
 
-template <typename In, typename Acc>
+template <typename In, typename Acc, int TILE = kTile, int STAGES = kStages>
 struct Ring {
+  using InT = In;
   using AccT = Acc;
+  static constexpr int kTile = TILE;
+  static constexpr int kStages = STAGES;
   In tile[kStages][kTile];
   Acc agg[kStages];
   Acc excl[kStages];
@@ -60,9 +63,9 @@ struct Ring {
 };
 
 // Thread 0, before the CTA's first barrier.
-template <typename In, typename Acc>
-__device__ __forceinline__ void init(Ring<In, Acc>& r, uint64_t limit_ns) {
-  for (int s = 0; s < kStages; ++s) {
+template <class R>
+__device__ __forceinline__ void init(R& r, uint64_t limit_ns) {
+  for (int s = 0; s < R::kStages; ++s) {
     mbar_init(&r.drawn[s], 1);
     mbar_init(&r.full[s], 1);
     mbar_init(&r.summed[s], 1);
@@ -89,14 +92,19 @@ __device__ __forceinline__ bool wait(R& r, uint64_t* bar, uint32_t parity, ScanH
 
 // Warp 0: for k = 0, 1, ... waits for stage k mod kStages to be free, draws
 // the next tile id and fills the stage with one bulk copy (the ragged last
-// tile with plain loads, zero-filled), then places `end_markers` end markers
+// tile zero-filled), then places `end_markers` end markers
 // (at least the number of warps of any role that takes alternate tiles, and
 // fewer than kStages).  The CTA
 // that draws the launch's last ticket (tiles + gridDim.x draws: every CTA
 // draws exactly one id past the end) resets the count and advances the epoch.
-template <typename In, typename Acc>
-__device__ void produce(Ring<In, Acc>& r, const In* __restrict__ x, int64_t n,
-                        unsigned int tiles, ScanHeader* hdr, int end_markers = kLookbackWarps) {
+// `first` (optional): the CTA's first ticket, already drawn; a ticket's tile
+// id is the ticket less `bias`.
+template <class R>
+__device__ void produce(R& r, const typename R::InT* x, int64_t n, unsigned int tiles,
+                        ScanHeader* hdr, int end_markers = kLookbackWarps,
+                        const unsigned long long* first = nullptr, unsigned int bias = 0u) {
+  using In = typename R::InT;
+  constexpr int kTile = R::kTile, kStages = R::kStages;
   const int lane = threadIdx.x & 31;
   const unsigned long long draws = static_cast<unsigned long long>(tiles) + gridDim.x;
   volatile int* abort_flag = &r.abort;
@@ -107,14 +115,17 @@ __device__ void produce(Ring<In, Acc>& r, const In* __restrict__ x, int64_t n,
     unsigned int tile = kEnd;
     if (ends == 0) {
       unsigned long long t = 0;
-      if (lane == 0) {
+      if (k == 0 && first) {
+        t = *first;
+      } else if (lane == 0) {
         t = atomicAdd(&hdr->ticket, 1ull);
         if (static_cast<unsigned int>(t) == draws - 1)
           atomicAdd(&hdr->ticket, (1ull << 32) - draws);
       }
       t = __shfl_sync(0xffffffffu, t, 0);
       if (k == 0 && lane == 0) r.epoch = t >> 32;
-      if (static_cast<unsigned int>(t) < tiles) tile = static_cast<unsigned int>(t);
+      const unsigned int id = static_cast<unsigned int>(t) - bias;
+      if (id < tiles) tile = id;
     }
     if (lane == 0) {
       r.ticket[s] = tile;
@@ -137,11 +148,27 @@ __device__ void produce(Ring<In, Acc>& r, const In* __restrict__ x, int64_t n,
         bulk_load(r.tile[s], x + base, kTile * sizeof(In), &r.full[s]);
       }
     } else {
-      for (int i = lane; i < kTile; i += 32) r.tile[s][i] = (base + i < n) ? x[base + i] : In(0);
+      // the ragged last tile: a bulk copy of its whole 16-byte units, a plain
+      // load of what is left, zeros behind (a loop of plain loads over the
+      // tile took the single warp some 17 us)
+      constexpr int kUnit = 16 / static_cast<int>(sizeof(In));
+      const int left = static_cast<int>(n - base), bulk = left / kUnit * kUnit;
+      static_assert(kTile % kUnit == 0, "a tile is whole 16-byte units");
+      if (lane < kUnit && bulk < left)
+        r.tile[s][bulk + lane] = bulk + lane < left ? x[base + bulk + lane] : In(0);
+      uint4* rest = reinterpret_cast<uint4*>(r.tile[s]) + (left + kUnit - 1) / kUnit;
+      const int units = (kTile - left) / kUnit;
+#pragma unroll 4
+      for (int i = lane; i < units; i += 32) rest[i] = make_uint4(0u, 0u, 0u, 0u);
       __syncwarp();
       if (lane == 0) {
         ++r.phases[s];
-        mbar_arrive(&r.full[s]);
+        if (bulk > 0) {
+          mbar_arrive_expect_tx(&r.full[s], bulk * sizeof(In));
+          bulk_load(r.tile[s], x + base, bulk * sizeof(In), &r.full[s]);
+        } else {
+          mbar_arrive(&r.full[s]);
+        }
       }
     }
   }
@@ -151,9 +178,11 @@ __device__ void produce(Ring<In, Acc>& r, const In* __restrict__ x, int64_t n,
 // starts when the tile id is drawn, walks back to the nearest inclusive
 // prefix, then, with the tile's aggregate, publishes its inclusive prefix and
 // hands the exclusive prefix to the compute warps.
-template <typename In, typename Acc>
-__device__ void look_back(Ring<In, Acc>& r, TileDesc* descs, Acc init, ScanHeader* hdr,
+template <class R>
+__device__ void look_back(R& r, TileDesc* descs, typename R::AccT init, ScanHeader* hdr,
                           int lw) {
+  using Acc = typename R::AccT;
+  constexpr int kStages = R::kStages;
   const int lane = threadIdx.x & 31;
   for (int k = lw;; k += kLookbackWarps) {
     const int s = k % kStages;
@@ -188,10 +217,10 @@ __device__ __forceinline__ void publish_aggregate(R& r, TileDesc* descs, int s,
 
 // Thread 0 after the CTA's final barrier: after an abort, bulk copies may
 // still be landing; wait (bounded) for the last phase started in each stage.
-template <typename In, typename Acc>
-__device__ __forceinline__ void drain(Ring<In, Acc>& r) {
+template <class R>
+__device__ __forceinline__ void drain(R& r) {
   if (!r.abort) return;
-  for (int s = 0; s < kStages; ++s)
+  for (int s = 0; s < R::kStages; ++s)
     if (r.phases[s] > 0u) mbar_wait_for(&r.full[s], (r.phases[s] - 1u) & 1u, r.limit_ns);
 }
 

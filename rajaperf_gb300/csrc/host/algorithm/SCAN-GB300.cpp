@@ -88,7 +88,8 @@ void SCAN::prepareRun(size_t tune_idx) {
                               reinterpret_cast<uintptr_t>(m_yi) % 16 == 0)
                            : (reinterpret_cast<uintptr_t>(m_x) % 16 == 0 &&
                               reinterpret_cast<uintptr_t>(m_y) % 16 == 0);
-  // the ring kernel (algo 0 for int64, 2 for FP64) is the one the stall targets
+  // the stall targets the ring kernel: algo 0 of int64, 2 of FP64 (whose algo 0
+  // is the tile kernel for short arrays)
   b200_tune tn = getTune(tune_idx);
   if (tn.algo == 2 || (tn.algo == 0 && isInt64(tune_idx))) tn.algo = 0;
   else if (tn.algo == 0) tn.algo = 1;
