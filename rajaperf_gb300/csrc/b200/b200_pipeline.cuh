@@ -90,6 +90,31 @@ __device__ __forceinline__ bool wait(R& r, uint64_t* bar, uint32_t parity, ScanH
   return ok;
 }
 
+// A whole warp fills a tile's stage with its `left` < TILE items and zeros
+// behind: a bulk copy of the whole 16-byte units, a plain load of what is left
+// (a loop of plain loads over the tile took the single warp some 17 us).
+template <typename In, int TILE>
+__device__ __forceinline__ void load_ragged(In* stage, const In* src, int left, uint64_t* full) {
+  constexpr int kUnit = 16 / static_cast<int>(sizeof(In));
+  static_assert(TILE % kUnit == 0, "a tile is whole 16-byte units");
+  const int lane = threadIdx.x & 31, bulk = left / kUnit * kUnit;
+  if (lane < kUnit && bulk < left)
+    stage[bulk + lane] = bulk + lane < left ? src[bulk + lane] : In(0);
+  uint4* rest = reinterpret_cast<uint4*>(stage) + (left + kUnit - 1) / kUnit;
+  const int units = (TILE - left) / kUnit;
+#pragma unroll 4
+  for (int i = lane; i < units; i += 32) rest[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+  if (lane == 0) {
+    if (bulk > 0) {
+      mbar_arrive_expect_tx(full, bulk * static_cast<uint32_t>(sizeof(In)));
+      bulk_load(stage, src, bulk * static_cast<uint32_t>(sizeof(In)), full);
+    } else {
+      mbar_arrive(full);
+    }
+  }
+}
+
 // Warp 0: for k = 0, 1, ... waits for stage k mod kStages to be free, draws
 // the next tile id and fills the stage with one bulk copy (the ragged last
 // tile zero-filled), then places `end_markers` end markers
@@ -148,28 +173,8 @@ __device__ void produce(R& r, const typename R::InT* x, int64_t n, unsigned int 
         bulk_load(r.tile[s], x + base, kTile * sizeof(In), &r.full[s]);
       }
     } else {
-      // the ragged last tile: a bulk copy of its whole 16-byte units, a plain
-      // load of what is left, zeros behind (a loop of plain loads over the
-      // tile took the single warp some 17 us)
-      constexpr int kUnit = 16 / static_cast<int>(sizeof(In));
-      const int left = static_cast<int>(n - base), bulk = left / kUnit * kUnit;
-      static_assert(kTile % kUnit == 0, "a tile is whole 16-byte units");
-      if (lane < kUnit && bulk < left)
-        r.tile[s][bulk + lane] = bulk + lane < left ? x[base + bulk + lane] : In(0);
-      uint4* rest = reinterpret_cast<uint4*>(r.tile[s]) + (left + kUnit - 1) / kUnit;
-      const int units = (kTile - left) / kUnit;
-#pragma unroll 4
-      for (int i = lane; i < units; i += 32) rest[i] = make_uint4(0u, 0u, 0u, 0u);
-      __syncwarp();
-      if (lane == 0) {
-        ++r.phases[s];
-        if (bulk > 0) {
-          mbar_arrive_expect_tx(&r.full[s], bulk * sizeof(In));
-          bulk_load(r.tile[s], x + base, bulk * sizeof(In), &r.full[s]);
-        } else {
-          mbar_arrive(&r.full[s]);
-        }
-      }
+      if (lane == 0) ++r.phases[s];
+      load_ragged<In, kTile>(r.tile[s], x + base, static_cast<int>(n - base), &r.full[s]);
     }
   }
 }

@@ -300,14 +300,10 @@ indexlist_pipelined(const double* __restrict__ x, int32_t* __restrict__ list, in
             mbar_arrive_expect_tx(&sm.full[d], kTile * sizeof(double));
             bulk_load(sm.tile[d], x + base, kTile * sizeof(double), &sm.full[d]);
           }
-        } else {  // the ragged last tile: plain loads, zero-filled (0 is not < 0)
-          for (int i = lane; i < kTile; i += 32)
-            sm.tile[d][i] = (base + i < n) ? x[base + i] : 0.0;
-          __syncwarp();
-          if (lane == 0) {
-            ++sm.phases[d];
-            mbar_arrive(&sm.full[d]);
-          }
+        } else {  // the ragged last tile, zero-filled (0 is not < 0)
+          if (lane == 0) ++sm.phases[d];
+          ring::load_ragged<double, kTile>(sm.tile[d], x + base, static_cast<int>(n - base),
+                                           &sm.full[d]);
         }
       }
       if (!ok) break;
