@@ -341,13 +341,14 @@ int b200_apps_del_dot_vec_2d(const double* x, const double* y,
 
 /* tsteps x (B <- 5-point average of A, then A <- of B) on an N x N grid
  *   -- polybench/POLYBENCH_JACOBI_2D.hpp:38-44, -Cuda.cpp:86-114
- * Default: column segments of tune->items rows per thread (2, 4 or 8;
- * default 4), the product by 0.2 and the first of each point's four adds on
- * the integer pipes (bit-identical: f64emu, exact rounding), the other three
- * adds on the FP64 pipe; tune->tile_z = 1 + integer-pipe adds per four
- * points (0, 4, 8, 9, 10 or 12; default 4), tune->tile_y 2 puts the product
- * on the FP64 pipe; tune->items 1: one point per
- * thread.  tune->algo > 0 selects the
+ * Default: each point's last two adds and the product by 0.2 in fixed point on
+ * the integer pipes (f64fix, exact rounding: bit-identical), the other two
+ * adds on the FP64 pipe; tune->items rows per thread (2, 4 or 8; by default 2
+ * or 3, by size).  tune->tile_y or tile_z choose a split by single operations
+ * instead (f64emu, bit-identical too; 4 rows by default): tune->tile_z = 1 +
+ * integer-pipe adds per four points (0, 4, 8, 9, 10 or 12; default 4),
+ * tune->tile_y 2 puts the product on the FP64 pipe; tune->items 1: one point
+ * per thread.  tune->algo > 0 selects the
  * mixed-pipe kernel: algo-1 of every 8 warps run bit-identical integer-pipe
  * FP64 (rows per warp: tile_y emulated, tile_z native).                     */
 int b200_polybench_jacobi_2d(double* A, double* B, int64_t N, int64_t tsteps,
@@ -355,7 +356,10 @@ int b200_polybench_jacobi_2d(double* A, double* B, int64_t N, int64_t tsteps,
 
 /* tsteps x (B <- 7-point heat update of A, then A <- of B) on N^3
  *   -- polybench/POLYBENCH_HEAT_3D.hpp:47-82, -Cuda.cpp:97-113
- * Default: each thread walks tune->tile_x consecutive planes (2 or 4;
+ * Default: directions i and j of each point in fixed point on the integer pipes
+ * (f64fix, exact rounding: bit-identical), direction k and the last two adds on
+ * the FP64 pipe.  With tune->tile_x or tile_z set, a split by single operations:
+ * each thread walks tune->tile_x consecutive planes (2 or 4;
  * default 4) with the plane neighbours in registers; 2.0 * a and the three
  * 0.125 * (...) are exponent moves, and tune->tile_z - 1 of the six
  * differences b(+1) - 2a of every two planes (0..6; default 5) run on the

@@ -11,8 +11,9 @@
 // into registers while the current one is consumed.  Each C element's dot
 // product runs over k in increasing order, as the suite's loop does.
 #include "b200_f64emu.cuh"
+#include "b200_f64fix.cuh"
 #include "b200_fma_form.cuh"
-#include "b200_internal.cuh"
+#include "b200_launch.cuh"
 
 #include <type_traits>
 
@@ -20,8 +21,12 @@ using namespace b200;
 
 namespace {
 
+// The kernels that launch() starts load coherently (b200_launch.cuh), with ld;
+// those launched plainly take the non-coherent path.
 template <typename T>
-__device__ __forceinline__ T ld(const T* p) { return __ldg(p); }
+__device__ __forceinline__ T ld(const T* p) { return *p; }
+template <typename T>
+__device__ __forceinline__ T ldnc(const T* p) { return __ldg(p); }
 
 // ---- JACOBI_2D: polybench/POLYBENCH_JACOBI_2D.hpp:38-44 ---------------------
 // One point per thread (tune->items 1).  The four adds stay on the FP64 pipe;
@@ -39,15 +44,15 @@ jacobi2d_step(const double* __restrict__ src, double* __restrict__ dst, int64_t 
        i += static_cast<int64_t>(gridDim.y) * BY) {
     const int64_t c = j + i * N;
     dst[c] = f64emu::mul_fast(
-        ld(src + c) + ld(src + c - 1) + ld(src + c + 1) + ld(src + c + N) + ld(src + c - N),
+        ldnc(src + c) + ldnc(src + c - 1) + ldnc(src + c + 1) + ldnc(src + c + N) + ldnc(src + c - N),
         0.2, slow);
   }
   if (__any_sync(__activemask(), slow) && slow) {
     for (int64_t i = 1 + static_cast<int64_t>(blockIdx.y) * BY + threadIdx.y; i < N - 1;
          i += static_cast<int64_t>(gridDim.y) * BY) {
       const int64_t c = j + i * N;
-      dst[c] = 0.2 * (ld(src + c) + ld(src + c - 1) + ld(src + c + 1) + ld(src + c + N) +
-                      ld(src + c - N));
+      dst[c] = 0.2 * (ldnc(src + c) + ldnc(src + c - 1) + ldnc(src + c + 1) + ldnc(src + c + N) +
+                      ldnc(src + c - N));
     }
   }
 }
@@ -83,11 +88,11 @@ jacobi2d_rows(const double* __restrict__ src, double* __restrict__ dst, int64_t 
   if (rows == R) {
     double col[R + 2], lft[R], rgt[R];
 #pragma unroll
-    for (int r = 0; r < R + 2; ++r) col[r] = ld(p + r * N);
+    for (int r = 0; r < R + 2; ++r) col[r] = ldnc(p + r * N);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      lft[r] = ld(p + (r + 1) * N - 1);
-      rgt[r] = ld(p + (r + 1) * N + 1);
+      lft[r] = ldnc(p + (r + 1) * N - 1);
+      rgt[r] = ldnc(p + (r + 1) * N + 1);
     }
     const fform::Regs fr = fform::regs(zero);
     const double fifth = fform::reg(0.2, zero);  // a per-thread register
@@ -108,6 +113,58 @@ jacobi2d_rows(const double* __restrict__ src, double* __restrict__ dst, int64_t 
     }
   }
   if (__any_sync(__activemask(), slow) && slow) {
+    for (int64_t r = 0; r < rows; ++r) {
+      const double* c = p + (r + 1) * N;
+      q[r * N] = 0.2 * (ldnc(c) + ldnc(c - 1) + ldnc(c + 1) + ldnc(c + N) + ldnc(c - N));
+    }
+  }
+}
+
+// The default.  As jacobi2d_rows, with the sums' last two adds and the product
+// by 0.2 in fixed point (b200_f64fix.cuh): the values of a thread's column are
+// unpacked once for the two points they are added to, and the FP64 pipe keeps
+// (c + l) + r, two register-operand FMAs per point instead of three.  Results
+// are bit for bit the suite's; a thread that met a value outside its window
+// redoes its points on the FP64 pipe after the loop.  Overlapped launches take
+// the gap between half-steps away.  Per half-step: 86.1 -> 75.8 us at 4002^2
+// (the integer ALU is the bound, 74 instructions a point), 10.3 -> 6.7 us at
+// 1002^2, 4.1 -> 1.8 us at 130^2.
+template <int BX, int R>
+__global__ void __launch_bounds__(BX)
+jacobi2d_fix(const double* src, double* dst, int64_t N, int zero) {
+  using namespace f64fix;
+  const int64_t j = 1 + static_cast<int64_t>(begin()) + static_cast<int64_t>(blockIdx.x) * BX +
+                    threadIdx.x;
+  if (j >= N - 1) return;
+  const int64_t i0 = 1 + static_cast<int64_t>(blockIdx.y) * R;
+  const int64_t rows = (N - 1 - i0 < R) ? (N - 1 - i0) : R;
+  const double* p = src + (i0 - 1) * N + j;
+  double* q = dst + i0 * N + j;
+  bool slow = rows < R;
+  if (!slow) {
+    double col[R + 2], lft[R], rgt[R], out[R];
+#pragma unroll
+    for (int r = 0; r < R + 2; ++r) col[r] = ld(p + r * N);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      lft[r] = ld(p + (r + 1) * N - 1);
+      rgt[r] = ld(p + (r + 1) * N + 1);
+    }
+    const fform::Regs fr = fform::regs(zero);
+    const Unit u = unit_at(col[1], 3, slow);
+    int64_t f[R + 2];
+#pragma unroll
+    for (int r = 0; r < R + 2; ++r) f[r] = fix(col[r], u, slow);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const double x = fform::add(fform::add(col[r + 1], lft[r], fr), rgt[r], fr);
+      const int64_t s = round53(round53(fix(x, u, slow) + f[r + 2]) + f[r]);
+      out[r] = pack_times(s, u, 0x1999999999999Aull, 1020);  // 0.2
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) q[r * N] = out[r];
+  }
+  if (slow) {
     for (int64_t r = 0; r < rows; ++r) {
       const double* c = p + (r + 1) * N;
       q[r * N] = 0.2 * (ld(c) + ld(c - 1) + ld(c + 1) + ld(c + N) + ld(c - N));
@@ -145,20 +202,20 @@ heat3d_step(const double* __restrict__ S, double* __restrict__ D, int64_t N, int
   bool slow = false;
   const double* p = S + k + N * (j + N * i0);
   double* q = D + k + N * (j + N * i0);
-  double im = ld(p - NN), a = ld(p);
+  double im = ldnc(p - NN), a = ldnc(p);
 #pragma unroll
   for (int r = 0; r < PL; ++r) {
     if (r >= np) break;
     const int ks = (KS2 * (r % 2 + 1)) / 2 - (KS2 * (r % 2)) / 2;  // this plane's share
-    const double ip = ld(p + NN);
+    const double ip = ldnc(p + NN);
     const double a2 = f64emu::mul_pow2_fast<1>(a, slow);
     auto dir = [&](int m, double hi, double lo) {
       const double d = (m < ks) ? f64emu::sub_near_fast(hi, a2, slow) : fform::sub(hi, a2, fr);
       return f64emu::mul_pow2_fast<-3>(fform::add(d, lo, fr), slow);
     };
     const double ti = dir(0, ip, im);
-    const double tj = dir(1, ld(p + N), ld(p - N));
-    const double tk = dir(2, ld(p + 1), ld(p - 1));
+    const double tj = dir(1, ldnc(p + N), ldnc(p - N));
+    const double tk = dir(2, ldnc(p + 1), ldnc(p - 1));
     *q = fform::add(fform::add(fform::add(ti, tj, fr), tk, fr), a, fr);
     im = a;
     a = ip;
@@ -168,6 +225,86 @@ heat3d_step(const double* __restrict__ S, double* __restrict__ D, int64_t N, int
   if (__any_sync(live, slow) && slow) {
     for (int r = 0; r < np; ++r) {
       const int64_t c = k + N * (j + N * (i0 + r));
+      const double a0 = ldnc(S + c);
+      D[c] = 0.125 * (ldnc(S + c + NN) - 2.0 * a0 + ldnc(S + c - NN)) +
+             0.125 * (ldnc(S + c + N) - 2.0 * a0 + ldnc(S + c - N)) +
+             0.125 * (ldnc(S + c + 1) - 2.0 * a0 + ldnc(S + c - 1)) + a0;
+    }
+  }
+}
+
+// The default.  A thread owns column (k, i) and walks PJ rows j.  The directions
+// i and j of a point, both differences, both sums and ti + tj, run in fixed
+// point (b200_f64fix.cuh): each value of the column is unpacked once for the
+// three points that use it, and the sums are rounded as they are, where
+// f64emu's adds unpack and pack every time.  Direction k and the last two adds
+// stay on the FP64 pipe: four register-operand FMAs per point (2 a and 0.125 x
+// are exact factors) where the kernel above issues 6.5; every FULL-th row also
+// runs direction k in fixed point, one FMA left.  Results are bit for bit the
+// suite's; a thread that met a value outside its window redoes its points on
+// the FP64 pipe after the loop.  One column and 64 registers per thread: two or
+// four columns save unpacking but leave too few warps to hide the loads.  Per
+// half-step (with the overlapped launches): 188 -> 108 us at 256^3 (FP64 pipe
+// and integer ALU both near 90%), 19.4 -> 11.1 us at 98^3, 8.3 -> 2.5 us at 32^3.
+template <int PJ, int FULL>
+__global__ void __launch_bounds__(256)
+heat3d_fix(const double* S, double* D, int64_t N, int zero) {
+  using namespace f64fix;
+  const int64_t k = 1 + static_cast<int64_t>(begin()) + static_cast<int64_t>(blockIdx.x) * 32 +
+                    threadIdx.x;
+  const int64_t j0 = 1 + static_cast<int64_t>(blockIdx.y) * PJ;
+  const int64_t i = 1 + static_cast<int64_t>(blockIdx.z) * 8 + threadIdx.y;
+  if (k >= N - 1 || i >= N - 1) return;
+  const int64_t NN = N * N;
+  const int rows = static_cast<int>((N - 1 - j0) < PJ ? (N - 1 - j0) : PJ);
+  const fform::Regs fr = fform::regs(zero);
+  const double mtwo = fform::reg(-2.0, zero), eighth = fform::reg(0.125, zero);
+  const double* p = S + k + N * (j0 + N * i);
+  double* q = D + k + N * (j0 + N * i);
+  bool slow = false;
+  // loads run one row ahead of the arithmetic: row j's value, row j + 1's, and
+  // row j's neighbours in k and i
+  double a = ld(p), an = ld(p + N), kp = ld(p + 1), km = ld(p - 1);
+  double ip = ld(p + NN), im = ld(p - NN);
+  const Unit u = unit_at(a, 4, slow);
+  int64_t fp = fix(ld(p - N), u, slow), fa = fix(a, u, slow);  // rows j - 1, j
+#pragma unroll FULL
+  for (int r = 0; r < rows; ++r) {
+    double an2, kp2, km2, ip2, im2;
+    if (r + 1 < rows) {
+      an2 = ld(p + 2 * N);
+      kp2 = ld(p + N + 1);
+      km2 = ld(p + N - 1);
+      ip2 = ld(p + N + NN);
+      im2 = ld(p + N - NN);
+    }
+    const int64_t fn = fix(an, u, slow);
+    const int64_t two = 2 * fa;
+    const int64_t ti = round53(round53(fix(ip, u, slow) - two) + fix(im, u, slow));
+    const int64_t tj = round53(round53(fn - two) + fp);
+    double t;
+    if (r % FULL == FULL - 1) {
+      const int64_t tk = round53(round53(fix(kp, u, slow) - two) + fix(km, u, slow));
+      t = pack(round53(ti + tj) + tk, u, -3);
+    } else {
+      const double tk = fform::add(fma(a, mtwo, kp), km, fr);
+      t = fma(tk, eighth, pack(ti + tj, u, -3));
+    }
+    *q = fform::add(t, a, fr);
+    a = an;
+    an = an2;
+    kp = kp2;
+    km = km2;
+    ip = ip2;
+    im = im2;
+    fp = fa;
+    fa = fn;
+    p += N;
+    q += N;
+  }
+  if (slow) {
+    for (int r = 0; r < rows; ++r) {
+      const int64_t c = k + N * (j0 + r + N * i);
       const double a0 = ld(S + c);
       D[c] = 0.125 * (ld(S + c + NN) - 2.0 * a0 + ld(S + c - NN)) +
              0.125 * (ld(S + c + N) - 2.0 * a0 + ld(S + c - N)) +
@@ -186,7 +323,7 @@ fdtd2d_e(double* __restrict__ ex, double* __restrict__ ey, const double* __restr
          const double* __restrict__ fict, int64_t t, int64_t nx, int64_t ny, int zero) {
   const int64_t j = static_cast<int64_t>(blockIdx.x) * BX + threadIdx.x;
   if (j >= ny) return;
-  const double f = ld(fict + t);
+  const double f = ldnc(fict + t);
   // register-operand FMAs (fform: the differences, and e - 0.5 d as the FMA
   // the compiler contracts it to, with -0.5 in a per-thread register), the
   // FP64 pipe's full-rate form; `zero` is 0 at run time
@@ -195,10 +332,10 @@ fdtd2d_e(double* __restrict__ ex, double* __restrict__ ey, const double* __restr
   for (int64_t i = static_cast<int64_t>(blockIdx.y) * BY + threadIdx.y; i < nx;
        i += static_cast<int64_t>(gridDim.y) * BY) {
     const int64_t c = j + i * ny;
-    const double h = ld(hz + c);
+    const double h = ldnc(hz + c);
     if (i == 0) ey[c] = f;
-    else ey[c] = fma(mhalf, fform::sub(h, ld(hz + c - ny), fr), ey[c]);
-    if (j >= 1) ex[c] = fma(mhalf, fform::sub(h, ld(hz + c - 1), fr), ex[c]);
+    else ey[c] = fma(mhalf, fform::sub(h, ldnc(hz + c - ny), fr), ey[c]);
+    if (j >= 1) ex[c] = fma(mhalf, fform::sub(h, ldnc(hz + c - 1), fr), ex[c]);
   }
 }
 
@@ -215,8 +352,8 @@ fdtd2d_h(const double* __restrict__ ex, const double* __restrict__ ey,
     const int64_t c = j + i * ny;
     // hz - 0.7 (((ex1 - ex0) + ey1) - ey0), left to right as the suite writes it
     hz[c] = fma(m07,
-                fform::sub(fform::add(fform::sub(ld(ex + c + 1), ld(ex + c), fr), ld(ey + c + ny), fr),
-                           ld(ey + c), fr),
+                fform::sub(fform::add(fform::sub(ldnc(ex + c + 1), ldnc(ex + c), fr), ldnc(ey + c + ny), fr),
+                           ldnc(ey + c), fr),
                 hz[c]);
   }
 }
@@ -244,6 +381,7 @@ constexpr int kFdtdMinRows = 8;    // the workspace holds snapshots for tiles th
 // 8192^2, 20 steps (GB300): 8 rows 0.965 ms per step (556 G FP64
 // instructions/s, 93% of the pipe), 16 rows 1.017, 32 rows 1.485 (the
 // two-launch form: 1.173); shorter tiles leave more CTAs resident per SM.
+// Overlapped launches: 50.4 -> 47.6 us per step at 2003 x 1501.
 constexpr int kFdtdDefaultRows = 8;
 
 struct FdtdSnap {
@@ -255,10 +393,13 @@ struct FdtdSnap {
   double* right_hz;  // [tile cols][nx]: hz of each tile's last column
 };
 
-__global__ void fdtd2d_snap_init(const double* __restrict__ ex, const double* __restrict__ ey,
-                                 const double* __restrict__ hz, int64_t nx, int64_t ny,
+__global__ void fdtd2d_snap_init(const double* ex, const double* ey, const double* hz, int64_t nx, int64_t ny,
                                  int64_t ntx, int64_t nty, int th, FdtdSnap s) {
   const int64_t nrow = nty * ny, total = nrow + ntx * nx;
+  const unsigned int z = begin();
+  ex += z;
+  ey += z;
+  hz += z;
   for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
        idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     if (idx < nrow) {
@@ -283,7 +424,7 @@ __global__ void fdtd2d_snap_init(const double* __restrict__ ex, const double* __
 template <int TH>
 __global__ void __launch_bounds__(kFdtdCols, (TH <= 8 ? 8 : TH <= 16 ? 5 : 3))
 fdtd2d_step_fused(double* __restrict__ ex, double* __restrict__ ey, double* __restrict__ hz,
-                  const double* __restrict__ fict, int64_t t, int64_t nx, int64_t ny,
+                  const double* fict, int64_t t, int64_t nx, int64_t ny,
                   FdtdSnap in, FdtdSnap out, int zero) {
   extern __shared__ __align__(16) double s_fdtd[];
   // new ex [rows][cols + 1] (column kFdtdCols: the right halo), new ey
@@ -295,6 +436,7 @@ fdtd2d_step_fused(double* __restrict__ ex, double* __restrict__ ey, double* __re
   double* sHzFirst = s_fdtd + TH * (kFdtdCols + 1) + (TH + 1) * kFdtdCols;
   double* sHzLast = sHzFirst + TH;
 
+  t += begin();
   const int tid = threadIdx.x, lane = tid & 31;
   const int64_t bx = blockIdx.x, by = blockIdx.y;
   const int64_t j0 = bx * kFdtdCols, i0 = by * TH;
@@ -425,11 +567,11 @@ int launch_fdtd_fused(double* ex, double* ey, double* hz, const double* fict, in
   const int64_t ntx = fdtd_tile_cols(ny), nty = fdtd_tile_rows(nx, TH);
   const int64_t total = nty * ny + ntx * nx;
   const unsigned ig = static_cast<unsigned>(std::min<int64_t>(ceil_div(total, 256), 4096));
-  fdtd2d_snap_init<<<ig, 256, 0, st>>>(ex, ey, hz, nx, ny, ntx, nty, TH, snap[0]);
+  launch(fdtd2d_snap_init, ig, 256, 0, st, ex, ey, hz, nx, ny, ntx, nty, TH, snap[0]);
   const dim3 g(static_cast<unsigned>(ntx), static_cast<unsigned>(nty));
   for (int64_t t = 0; t < tsteps; ++t)
-    fdtd2d_step_fused<TH><<<g, kFdtdCols, fdtd_smem(TH), st>>>(ex, ey, hz, fict, t, nx, ny,
-                                                               snap[t & 1], snap[(t + 1) & 1], 0);
+    launch(fdtd2d_step_fused<TH>, g, kFdtdCols, fdtd_smem(TH), st, ex, ey, hz, fict, t, nx, ny,
+           snap[t & 1], snap[(t + 1) & 1], 0);
   return B200_OK;
 }
 
@@ -459,11 +601,11 @@ __device__ __forceinline__ void jacobi_rows(const double* __restrict__ S, double
                                             int64_t N, int64_t j, int64_t i_first, int rows) {
   if (i_first >= N - 1) return;  // this warp's rows lie past the interior
   int64_t c = j + i_first * N;
-  double up = ld(S + c - N), mid = ld(S + c);
+  double up = ldnc(S + c - N), mid = ldnc(S + c);
   for (int r = 0; r < rows; ++r, c += N) {
     if (i_first + r >= N - 1) break;
-    const double down = ld(S + c + N);
-    D[c] = jacobi_pt<EMU>(mid, ld(S + c - 1), ld(S + c + 1), down, up);
+    const double down = ldnc(S + c + N);
+    D[c] = jacobi_pt<EMU>(mid, ldnc(S + c - 1), ldnc(S + c + 1), down, up);
     up = mid;
     mid = down;
   }
@@ -512,10 +654,10 @@ __device__ __forceinline__ void heat_rows(const double* __restrict__ S, double* 
     const int64_t j = j_first + r;
     if (j >= N - 1) break;
     int64_t c = k + N * (j + N * i0);
-    double im = ld(S + c - NN), a = ld(S + c);
+    double im = ldnc(S + c - NN), a = ldnc(S + c);
     for (int64_t i = i0; i < i0 + ni && i < N - 1; ++i, c += NN) {
-      const double ip = ld(S + c + NN);
-      D[c] = heat_pt<EMU>(a, ip, im, ld(S + c + N), ld(S + c - N), ld(S + c + 1), ld(S + c - 1));
+      const double ip = ldnc(S + c + NN);
+      D[c] = heat_pt<EMU>(a, ip, im, ldnc(S + c + N), ldnc(S + c - N), ldnc(S + c + 1), ldnc(S + c - 1));
       im = a;
       a = ip;
     }
@@ -580,9 +722,9 @@ dgemm_kernel(const double* __restrict__ A, const double* __restrict__ B,
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       int64_t gi = i0 + la_i + r * 16, gk = k0 + la_k;
-      ra[r] = (gi < ni && gk < nk) ? ld(A + gk + gi * nk) : 0.0;
+      ra[r] = (gi < ni && gk < nk) ? ldnc(A + gk + gi * nk) : 0.0;
       int64_t gk2 = k0 + lb_k + r * 4, gj = j0 + lb_j;
-      rb[r] = (gk2 < nk && gj < nj) ? ld(B + gj + gk2 * nj) : 0.0;
+      rb[r] = (gk2 < nk && gj < nj) ? ldnc(B + gj + gk2 * nj) : 0.0;
     }
   };
   load(0);
@@ -644,7 +786,7 @@ dim3 grid2(int64_t nxthreads, int64_t nrows, int bx, int by) {
 
 extern "C" {
 
-// JACOBI_2D's split between the pipes by default: integer-pipe adds per
+// JACOBI_2D's explicit split between the pipes: integer-pipe adds per
 // four points and where the product by 0.2 runs.  Measured on GB300 (4 rows
 // per thread, us per half-step at 4096^2): FP64 adds only 114.7; one add per
 // point on the integer pipe 92.3; two 125.1; with the product on the FP64
@@ -656,7 +798,7 @@ extern "C" {
 constexpr int kJacobiIntAdds4 = 4;
 constexpr bool kJacobiMulInt = true;
 
-// HEAT_3D by default: planes per thread and integer-pipe differences
+// HEAT_3D's explicit split: planes per thread and integer-pipe differences
 // b(+1) - 2a per two planes.  Measured on GB300 (us per half-step at 256^3,
 // 4 planes): 0 of 6 on the integer pipes 243.9, 2: 219.2, 4: 194.7,
 // 5: 184.8, 6: 217.2 (the integer ALU 88% busy: each such difference costs
@@ -666,6 +808,11 @@ constexpr bool kJacobiMulInt = true;
 // cancels leaves the close-exponent form).
 constexpr int kHeatPlanes = 4;
 constexpr int kHeatIntSubs2 = 5;
+// The fixed-point kernel, the default: every how many rows direction k runs in
+// fixed point too, which puts the integer ALU and the FP64 pipe level (us per
+// half-step at 256^3: never 117, every 8th 114, 4th 108, 3rd 108, 2nd 112).
+constexpr int kHeatFixThreads = 1024;
+constexpr int kHeatFull = 4;
 
 int b200_polybench_jacobi_2d(double* A, double* B, int64_t N, int64_t tsteps,
                              const b200_tune* tune, b200_stream_t stream) {
@@ -684,9 +831,37 @@ int b200_polybench_jacobi_2d(double* A, double* B, int64_t N, int64_t tsteps,
     }
     return after_launch("b200_polybench_jacobi_2d", static_cast<int>(2 * tsteps));
   }
-  // default: column segments of 4 rows per thread (tune->items 2, 4 or 8);
+  const int items = tune ? tune->items : 0;
+  const bool split = tune && (tune->tile_y != 0 || tune->tile_z != 0);
+  if (!split && (items == 0 || items == 2 || items == 4 || items == 8)) {
+    constexpr int BX = 128;
+    auto run = [&](auto rows_tag) -> int {
+      constexpr int R = decltype(rows_tag)::value;
+      const int64_t gy = ceil_div(N - 2, R);
+      if (gy > 65535) return invalid("b200_polybench_jacobi_2d: N too large for %d rows", R);
+      const dim3 g(static_cast<unsigned>(ceil_div(N - 2, BX)), static_cast<unsigned>(gy));
+      for (int64_t t = 0; t < tsteps; ++t) {
+        launch(jacobi2d_fix<BX, R>, g, BX, 0, st, A, B, N, 0);
+        launch(jacobi2d_fix<BX, R>, g, BX, 0, st, B, A, N, 0);
+      }
+      return B200_OK;
+    };
+    // Rows per thread, 2 or 3 (us per half-step): 3.94 or 4.96 at N = 600, 5.27
+    // or 5.16 at 800, 83.8 or 75.8 at 4002; 4 rows 76.5 there and 6.79 at 1002
+    // against 6.69.  Three from 1536 threads of two rows per SM on.
+    const double per_sm = static_cast<double>(N - 2) * (N - 2) / device_info().sm_count;
+    const int R = items ? items : (per_sm / 2 < 1536 ? 2 : 3);
+    const int rc = R == 2   ? run(std::integral_constant<int, 2>{})
+                   : R == 3 ? run(std::integral_constant<int, 3>{})
+                   : R == 4 ? run(std::integral_constant<int, 4>{})
+                            : run(std::integral_constant<int, 8>{});
+    if (rc != B200_OK) return rc;
+    return after_launch("b200_polybench_jacobi_2d", static_cast<int>(2 * tsteps));
+  }
+  // an explicit split: column segments of 4 rows per thread (tune->items 2, 4
+  // or 8);
   // tune->items 1: one point per thread with rows strided over the grid
-  const int rows = (tune && tune->items) ? tune->items : 4;
+  const int rows = items ? items : 4;
   if (rows != 1 && rows != 2 && rows != 4 && rows != 8)
     return invalid("b200_polybench_jacobi_2d: items %d (1, 2, 4 or 8)", rows);
   if (rows != 1) {
@@ -756,6 +931,33 @@ int b200_polybench_heat_3d(double* A, double* B, int64_t N, int64_t tsteps,
       heat3d_mixed<<<g, 256, 0, st>>>(A, B, N, m, chunk);
       heat3d_mixed<<<g, 256, 0, st>>>(B, A, N, m, chunk);
     }
+    return after_launch("b200_polybench_heat_3d", static_cast<int>(2 * tsteps));
+  }
+  if (!tune || (tune->tile_x <= 0 && tune->tile_z <= 0)) {
+    auto run = [&](auto rows_tag) -> int {
+      constexpr int PJ = decltype(rows_tag)::value;
+      const int64_t gy = ceil_div(N - 2, PJ), gz = ceil_div(N - 2, 8);
+      if (gy > 65535 || gz > 65535) return invalid("b200_polybench_heat_3d: N too large");
+      const dim3 g(static_cast<unsigned>(ceil_div(N - 2, 32)), static_cast<unsigned>(gy),
+                   static_cast<unsigned>(gz));
+      for (int64_t t = 0; t < tsteps; ++t) {
+        launch(heat3d_fix<PJ, kHeatFull>, g, dim3(32, 8), 0, st, A, B, N, 0);
+        launch(heat3d_fix<PJ, kHeatFull>, g, dim3(32, 8), 0, st, B, A, N, 0);
+      }
+      return B200_OK;
+    };
+    // rows per thread: as many as leave every SM kHeatFixThreads threads (1, 2,
+    // 4, 8, 16 rows, us per half-step: N = 258: 199, 157, 132, 122, 119; N = 100:
+    // 14.0, 12.4, 11.7, 12.7, 19.5; N = 34: 2.5, 2.8, 3.5, 5.2, 8.5)
+    const double per_sm = static_cast<double>(N - 2) * (N - 2) * (N - 2) / device_info().sm_count;
+    int pj = 16;
+    while (pj > 1 && per_sm / pj < kHeatFixThreads) pj /= 2;
+    const int rc = pj == 16  ? run(std::integral_constant<int, 16>{})
+                   : pj == 8 ? run(std::integral_constant<int, 8>{})
+                   : pj == 4 ? run(std::integral_constant<int, 4>{})
+                   : pj == 2 ? run(std::integral_constant<int, 2>{})
+                             : run(std::integral_constant<int, 1>{});
+    if (rc != B200_OK) return rc;
     return after_launch("b200_polybench_heat_3d", static_cast<int>(2 * tsteps));
   }
   constexpr int BX = 32, BY = 8;
