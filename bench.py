@@ -1040,9 +1040,10 @@ def measure_gemm_suite_shape(torch, rp, stream, n, seed):
 
 def measure_3mm(torch, rp, stream, n=2048, seed=4793):
     """Polybench 3MM, square N: E = A*B, F = C*D, G = E*F with entries uniform
-    in [-1, 1); native FP64 (b200_polybench_3mm) against three split-precision
-    products (b200_gemm_split, alpha 1, beta 0), TFLOP/s at 3 * 2 N^3 and the
-    split G's relative Frobenius error against the native G."""
+    in [-1, 1); native FP64 (b200_polybench_3mm on the FP64 pipe) against its
+    default and three split-precision products (b200_gemm_split, alpha 1, beta
+    0), TFLOP/s at 3 * 2 N^3 and the split G's relative Frobenius error against
+    the native G."""
     L = rp.b200()
     s = stream.cuda_stream
     g = torch.Generator(device="cuda").manual_seed(seed + 3 * n)
@@ -1054,9 +1055,15 @@ def measure_3mm(torch, rp, stream, n=2048, seed=4793):
     ws = torch.zeros(wb, dtype=torch.uint8, device="cuda")
     P = lambda t: t.data_ptr()
 
-    def native():
+    fp64_pipe = rp.Tune(algo=1)
+
+    def default():
         return L.b200_polybench_3mm(P(A), P(B), P(C), P(D), P(E), P(F), P(G), n, n, n, n, n,
                                     None, s)
+
+    def native():
+        return L.b200_polybench_3mm(P(A), P(B), P(C), P(D), P(E), P(F), P(G), n, n, n, n, n,
+                                    ctypes.byref(fp64_pipe), s)
 
     def split():
         for x, y, z in ((A, B, Es), (C, D, Fs), (Es, Fs, Gs)):
@@ -1066,7 +1073,7 @@ def measure_3mm(torch, rp, stream, n=2048, seed=4793):
         return 0
 
     res = {"n": n}
-    for name, fn in (("native", native), ("split", split)):
+    for name, fn in (("default", default), ("native", native), ("split", split)):
         rp.check(fn(), name)  # warm-up
         best = None
         for _ in range(3):

@@ -48,6 +48,7 @@
 // offset 16 of the workspace and the CTA winds down.
 #include "b200_internal.cuh"
 #include "b200_async.cuh"
+#include "b200_tcgen05.cuh"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -405,6 +406,8 @@ __global__ void __launch_bounds__(256, 1) ozaki_mma_kernel(SplitArgs g) {
 // ---- tcgen05 engine ------------------------------------------------------------
 namespace tc {
 
+using namespace tcgen05;
+
 constexpr int BM = 128, BN = 128;
 constexpr int kRowBytes = 128;                      // one 128-byte swizzle row of K
 // k values per k block: 64 bf16 or 128 e4m3 (one swizzle row either way)
@@ -428,28 +431,6 @@ template <bool F8>
 constexpr uint32_t kIdesc = F8 ? kIdescShape : (kIdescShape | (1u << 7) | (1u << 10));
 static_assert(kSmemBytes <= 232448, "shared memory budget");
 
-// Waits for the phase of parity `parity` to complete.  Gives up after
-// limit_ns (setting the CTA's abort flag) or when another role has aborted.
-__device__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag,
-                          uint64_t limit_ns) {
-  if (mbar_try_wait(b, parity)) return true;
-  const uint64_t t0 = globaltimer();
-  for (;;) {
-    if (mbar_try_wait(b, parity)) return true;
-    if (*abort_flag) return false;
-    if (globaltimer() - t0 > limit_ns) {
-      *abort_flag = 1;
-      return false;
-    }
-  }
-}
-// The same wait for the wind-down after an abort: bounded, ignores the flag.
-__device__ bool mbar_wait_drain(uint64_t* b, uint32_t parity, uint64_t limit_ns) {
-  const uint64_t t0 = globaltimer();
-  while (!mbar_try_wait(b, parity))
-    if (globaltimer() - t0 > limit_ns) return false;
-  return true;
-}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar,
                                             int x, int y) {
   asm volatile(
@@ -457,20 +438,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-// K-major operand tile of 8-row x 128-byte swizzle atoms (as TMA's 128-byte
-// swizzle writes it): start >> 4, leading offset 16 B (unused for this
-// layout), stride 1024 B between 8-row groups, descriptor version 1,
-// swizzle mode 2 (128 B).
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-  return static_cast<uint64_t>((saddr >> 4) & 0x3FFFu) | (1ull << 16) |
-         (static_cast<uint64_t>(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 // One 128 x 128 x (32 bytes of K) MMA: 16 bf16 (kind::f16) or 32 e4m3
 // (kind::f8f6f4) values of k, FP32 accumulation in tensor memory.
@@ -492,51 +459,6 @@ __device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t adesc, uint64_t b
         "l"(adesc), "l"(bdesc), "r"(kIdesc<false>), "r"(accumulate)
         : "memory");
   }
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-        "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
-// tcgen05.wait::ld, tied to the loaded registers so that no use of them is
-// scheduled before the wait.
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
-                 "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
-                 "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-               :
-               : "memory");
-}
-__device__ __forceinline__ void tmem_keep(uint32_t (&r)[16]) {
-  asm volatile(""
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
-                 "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
-                 "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-               :
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
-      "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() {
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ double pair_to_double(uint32_t lo, uint32_t hi) {
   return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));

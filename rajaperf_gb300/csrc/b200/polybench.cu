@@ -10,6 +10,7 @@
 // accumulators per thread, K in steps of 16 with the next K slice prefetched
 // into registers while the current one is consumed.  Each C element's dot
 // product runs over k in increasing order, as the suite's loop does.
+#include "b200_dgemm.cuh"
 #include "b200_f64emu.cuh"
 #include "b200_f64fix.cuh"
 #include "b200_fma_form.cuh"
@@ -1074,8 +1075,16 @@ int b200_polybench_3mm(const double* A, const double* B, const double* C,
   if (!A || !B || !C || !D || !E || !F || !G || ni < 0 || nj < 0 || nk < 0 || nl < 0 ||
       nm < 0)
     return invalid("b200_polybench_3mm: bad args");
-  (void)tune;
   cudaStream_t st = as_stream(stream);
+  const Product p[3] = {{A, B, E, ni, nj, nk}, {C, D, F, nj, nl, nm}, {E, F, G, ni, nl, nj}};
+  // tune->algo 1: the FP64 pipe
+  if (!(tune && tune->algo == 1) && dgemm_tc_takes(p[0]) && dgemm_tc_takes(p[1]) &&
+      dgemm_tc_takes(p[2])) {
+    int s = launch_dgemm_tc(p, 2, st);
+    if (s == B200_OK) s = launch_dgemm_tc(p + 2, 1, st);
+    if (s != B200_OK) return s;
+    return after_launch("b200_polybench_3mm", 2);
+  }
   int s = launch_dgemm(A, B, E, ni, nj, nk, 1.0, 0.0, 0, st);   // E = A*B
   if (s == B200_OK) s = launch_dgemm(C, D, F, nj, nl, nm, 1.0, 0.0, 0, st);  // F = C*D
   if (s == B200_OK) s = launch_dgemm(E, F, G, ni, nl, nj, 1.0, 0.0, 0, st);  // G = E*F
