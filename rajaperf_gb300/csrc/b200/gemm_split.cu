@@ -24,9 +24,10 @@
 // tests and bench.  The e4m3 and bf16 slices hold the same digits, so the
 // engines' results agree bit for bit whenever the accumulation is exact.
 //
-// Engines (tune->algo; 0 picks 4):
+// Engines (tune->algo; 0 picks the resident-weights engine for the default 10
+// slices and k <= 8192, see there, and 4 elsewhere):
 //  4 tcgen05 on e4m3 slices with the digit weights in pairs (128 x 256 MMAs;
-//    see the paired-weight engine below): the default.
+//    see the paired-weight engine below).
 //  3 tcgen05 on e4m3 slices, 2 the same on bf16 slices: one 128x128 C tile
 //    per CTA (CTAs ordered in groups of 8 tile rows, so that resident CTAs
 //    share operand tiles in L2).  Warp 0 streams 128 x (128 bytes of k) slice
@@ -48,6 +49,7 @@
 // offset 16 of the workspace and the CTA winds down.
 #include "b200_internal.cuh"
 #include "b200_async.cuh"
+#include "b200_f64fix.cuh"
 #include "b200_tcgen05.cuh"
 
 #include <cuda.h>
@@ -130,18 +132,11 @@ col_max_kernel(const double* __restrict__ B, int64_t K, int64_t N,
 // [-0.52, 0.49] * 32^(S-1)); the top digit takes what is left, an integer of
 // magnitude below 16.52, so |d_0| <= 16.
 
-// Digit e (0-based) of a 16-byte word of slice digits in the arrays'
-// storage type: e4m3 bytes (exact for the integers |d| <= 16) or bf16.
+// Digit e (0-based) of a 16-byte word of slice digits as bf16.
 template <typename T>
 __device__ __forceinline__ void pack_digit(uint32_t (&w)[4], int e, int d) {
-  if constexpr (sizeof(T) == 1) {
-    const uint32_t b = static_cast<uint32_t>(
-        __nv_cvt_float_to_fp8(static_cast<float>(d), __NV_SATFINITE, __NV_E4M3));
-    w[e >> 2] |= b << (8 * (e & 3));
-  } else {
-    const uint32_t h = __bfloat16_as_ushort(__float2bfloat16_rn(static_cast<float>(d)));
-    w[e >> 1] |= h << (16 * (e & 1));
-  }
+  const uint32_t h = __bfloat16_as_ushort(__float2bfloat16_rn(static_cast<float>(d)));
+  w[e >> 1] |= h << (16 * (e & 1));
 }
 
 // The S digits of q = round(v * 2^shift) (as digits_of), slice s into w[s]
@@ -161,10 +156,62 @@ __device__ __forceinline__ void put_digits(double v, int shift, int S, int e,
   pack_digit<T>(w[0], e, static_cast<int>(q));
 }
 
+// round(v * 2^shift) to nearest even on the integer pipes, as
+// __double2ll_rn(scalbn(v, shift)) has it (magnitudes below 2^60).
+__device__ __forceinline__ long long scaled_round(double v, int shift) {
+  const uint64_t b = f64emu::bits_opaque(v);
+  const int e = static_cast<int>(b >> 52) & 0x7ff;
+  if (e == 0x7ff) return __double2ll_rn(scalbn(v, shift));
+  const uint64_t m = (b & f64emu::kFrac) | (e ? f64emu::kHidden : 0ull);
+  const int x = (e ? e : 1) - 1075 + shift;  // v * 2^shift = m * 2^x
+  const int r = x < 0 ? (x > -63 ? -x : 63) : 0;
+  const uint64_t kept = m >> r;
+  const uint64_t half = r ? (1ull << (r - 1)) - 1u + (kept & 1u) : 0u;
+  const uint64_t q = ((m + half) >> r) << (x > 0 ? x : 0);
+  return (b >> 63) ? -static_cast<long long>(q) : static_cast<long long>(q);
+}
+
+// The e4m3 codes of the integers u0 - 16 and u1 - 16 (|.| <= 16), in the low
+// and high byte: 1024 + u as f16s, minus 1040, converted together.
+__device__ __forceinline__ uint32_t codes2(uint32_t u0, uint32_t u1) {
+  uint32_t h = u0 | (u1 << 16) | 0x64006400u;
+  uint16_t c;
+  asm("{\n\t.reg .b32 t;\n\t"
+      "sub.f16x2 t, %1, %2;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f16x2 %0, t;\n\t}"
+      : "=h"(c)
+      : "r"(h), "r"(0x64106410u));
+  return c;
+}
+
+// q + 16 (1 + 32 + .. + 32^(S-2)): its 5-bit fields are the balanced digits
+// plus 16, what is left above them the top digit.
+__device__ __forceinline__ uint64_t biased(long long q, int S) {
+  constexpr uint64_t kSixteens = 0x0842108421084210ull;  // 16 in every 5-bit field
+  return static_cast<uint64_t>(q) + (kSixteens & ((1ull << (kSliceBits * (S - 1))) - 1u));
+}
+__device__ __forceinline__ uint32_t field(uint64_t t, int s, int S) {
+  const uint32_t v = static_cast<uint32_t>(static_cast<long long>(t) >> (kSliceBits * (S - 1 - s)));
+  return s == 0 ? v + 16u : v & 31u;
+}
+
+// Byte offset of the 16-byte word of slice s (of S), row `row` (of `rows`) and
+// bytes k0 .. k0 + 15 of K in a slice array: rows of K (the tensor maps' view),
+// or, for the resident engine, blocks of 64 bytes of K, in each block the
+// slices, in each slice all rows as the 64-byte swizzle wants them in shared
+// memory, so that a tile's rows are one contiguous piece.
+template <bool BLOCKED>
+__device__ __forceinline__ int64_t word_offset(int s, int S, int64_t row, int64_t rows,
+                                               int64_t row_bytes, int64_t k0) {
+  if (!BLOCKED) return (s * rows + row) * row_bytes + k0;
+  const int64_t unit = (k0 >> 4) & 3;
+  return (((k0 >> 6) * S + s) * rows + row) * 64 + ((unit ^ ((row >> 1) & 3)) << 4);
+}
+
 // As[s][i][k] (Mp x Kp, zero padded) from A (M x K): a thread forms the digits
 // of 16 bytes' worth of consecutive k of one row (16 e4m3 or 8 bf16 digits
 // per slice) and writes one 16-byte word to every slice.
-template <typename T>
+template <typename T, bool BLOCKED>
 __global__ void __launch_bounds__(128)
 slice_a_kernel(const double* __restrict__ A, int64_t M, int64_t K, const int* __restrict__ E,
                int S, int64_t Mp, int64_t Kp, T* __restrict__ As) {
@@ -177,16 +224,31 @@ slice_a_kernel(const double* __restrict__ A, int64_t M, int64_t K, const int* __
   uint32_t w[kMaxSlices][4];
 #pragma unroll
   for (int s = 0; s < kMaxSlices; ++s) w[s][0] = w[s][1] = w[s][2] = w[s][3] = 0u;
+  if constexpr (sizeof(T) == 1) {
 #pragma unroll
-  for (int e = 0; e < kPer; ++e) {
-    const int64_t k = k0 + e;
-    const double v = (row && k < K) ? __ldg(A + i * K + k) : 0.0;
-    put_digits<T>(v, shift, S, e, w);
+    for (int e = 0; e < kPer; e += 2) {
+      const double v0 = (row && k0 + e < K) ? __ldg(A + i * K + k0 + e) : 0.0;
+      const double v1 = (row && k0 + e + 1 < K) ? __ldg(A + i * K + k0 + e + 1) : 0.0;
+      const uint64_t t0 = biased(scaled_round(v0, shift), S);
+      const uint64_t t1 = biased(scaled_round(v1, shift), S);
+#pragma unroll
+      for (int s = 0; s < kMaxSlices; ++s)
+        if (s < S) w[s][e >> 2] |= codes2(field(t0, s, S), field(t1, s, S)) << (8 * (e & 2));
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      const int64_t k = k0 + e;
+      const double v = (row && k < K) ? __ldg(A + i * K + k) : 0.0;
+      put_digits<T>(v, shift, S, e, w);
+    }
   }
 #pragma unroll
   for (int s = 0; s < kMaxSlices; ++s)
     if (s < S)
-      *reinterpret_cast<uint4*>(As + (s * Mp + i) * Kp + k0) =
+      *reinterpret_cast<uint4*>(
+          reinterpret_cast<char*>(As) +
+          word_offset<BLOCKED>(s, S, i, Mp, Kp * sizeof(T), k0 * sizeof(T))) =
           make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
 }
 
@@ -196,7 +258,7 @@ slice_a_kernel(const double* __restrict__ A, int64_t M, int64_t K, const int* __
 // leave as 16-byte words along Bt's rows.  The CTAs of the first k tile also
 // write the column exponents Eb from the column maxima.
 constexpr int kBtK = 32, kBtJ = 64;
-template <typename T>
+template <typename T, bool BLOCKED>
 __global__ void __launch_bounds__(256)
 slice_b_kernel(const double* __restrict__ B, int64_t K, int64_t N,
                const unsigned long long* __restrict__ bmax, int* __restrict__ Eb, int S,
@@ -221,30 +283,58 @@ slice_b_kernel(const double* __restrict__ B, int64_t K, int64_t N,
   const int jj = tid & (kBtJ - 1);
   const int64_t j = j0 + jj;
   const int shift = kSliceBits * S - sE[jj];
+  if constexpr (sizeof(T) == 1) {  // the digits' codes, two k at a time
 #pragma unroll 2
-  for (int r = 0; r < kBtK / 4; ++r) {
-    const int kk = (tid >> 6) + 4 * r;
-    const int64_t k = k0 + kk;
-    const double v = (k < K && j < N) ? __ldg(B + k * N + j) : 0.0;
-    long long q = __double2ll_rn(scalbn(v, shift));
+    for (int r = 0; r < kBtK / 4; r += 2) {
+      const int kk = (tid >> 6) + 4 * r;
+      const int64_t k = k0 + kk;
+      const double v0 = (k < K && j < N) ? __ldg(B + k * N + j) : 0.0;
+      const double v1 = (k + 4 < K && j < N) ? __ldg(B + (k + 4) * N + j) : 0.0;
+      const uint64_t t0 = biased(scaled_round(v0, shift), S);
+      const uint64_t t1 = biased(scaled_round(v1, shift), S);
 #pragma unroll
-    for (int s = kMaxSlices - 1; s >= 1; --s) {
-      if (s < S) {
-        const long long d = ((q + 16) & 31) - 16;
-        dig[s][jj][kk] = static_cast<signed char>(d);
-        q = (q - d) >> kSliceBits;
+      for (int s = 0; s < kMaxSlices; ++s) {
+        if (s < S) {
+          const uint32_t c = codes2(field(t0, s, S), field(t1, s, S));
+          dig[s][jj][kk] = static_cast<signed char>(c);
+          dig[s][jj][kk + 4] = static_cast<signed char>(c >> 8);
+        }
       }
     }
-    dig[0][jj][kk] = static_cast<signed char>(q);
+  } else {
+#pragma unroll 2
+    for (int r = 0; r < kBtK / 4; ++r) {
+      const int kk = (tid >> 6) + 4 * r;
+      const int64_t k = k0 + kk;
+      const double v = (k < K && j < N) ? __ldg(B + k * N + j) : 0.0;
+      long long q = __double2ll_rn(scalbn(v, shift));
+#pragma unroll
+      for (int s = kMaxSlices - 1; s >= 1; --s) {
+        if (s < S) {
+          const long long d = ((q + 16) & 31) - 16;
+          dig[s][jj][kk] = static_cast<signed char>(d);
+          q = (q - d) >> kSliceBits;
+        }
+      }
+      dig[0][jj][kk] = static_cast<signed char>(q);
+    }
   }
   __syncthreads();
   for (int c = tid; c < S * kBtJ * kChunks; c += 256) {
     const int s = c / (kBtJ * kChunks), rem = c % (kBtJ * kChunks);
     const int row = rem / kChunks, ch = rem % kChunks;
     uint32_t w[4] = {0u, 0u, 0u, 0u};
+    if constexpr (sizeof(T) == 1) {
 #pragma unroll
-    for (int e = 0; e < kPer; ++e) pack_digit<T>(w, e, dig[s][row][ch * kPer + e]);
-    *reinterpret_cast<uint4*>(Bt + (s * Np + j0 + row) * Kp + k0 + ch * kPer) =
+      for (int e = 0; e < 4; ++e)
+        w[e] = *reinterpret_cast<const uint32_t*>(&dig[s][row][ch * kPer + 4 * e]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < kPer; ++e) pack_digit<T>(w, e, dig[s][row][ch * kPer + e]);
+    }
+    *reinterpret_cast<uint4*>(
+        reinterpret_cast<char*>(Bt) +
+        word_offset<BLOCKED>(s, S, j0 + row, Np, Kp * sizeof(T), (k0 + ch * kPer) * sizeof(T))) =
         make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
@@ -974,6 +1064,231 @@ ozaki_tc_paired_kernel(const __grid_constant__ CUtensorMap tmA,
   }
 }
 
+// ---- resident-weights engine -----------------------------------------------------
+// The engines above stream the operands of every digit weight anew: a 128 x 256
+// MMA's 48 KB serve 512 tensor cycles, and the tensor pipe waits for the L2.
+// Here a CTA owns a 128 x 48 tile, whose sums of all S <= 10 weights fit in
+// tensor memory at once (S x 48 FP32 columns), so each slice of a k block is
+// loaded once and meets every slice it has to: 55 KB serve 1425 tensor cycles
+// of S = 10.  The B slices of a block stand one under the other, so that
+// A_s * [B_1; ..; B_(S+1-s)] is one MMA (two above 240 columns) into columns
+// 48 (s - 1) .. of the sums.  Blocks are 64 bytes of k (64-byte swizzle), two
+// stages of 110 KB.  The slices are laid out for it (word_offset), so that a
+// stage is 20 contiguous bulk copies: tensor maps' boxes of 64-byte rows moved a
+// third of that (3426 us at 3500 x 3500 x 4200).
+// The epilogue folds the weights in the other engines' order and with their
+// roundings, on the integer pipes as far as 64 bits reach: the sums of weights
+// 2 .. 8 are exact in 53 bits, 9 and 10 are rounded in place (f64fix::round53),
+// and 11 as the sum is packed, or by an FP64 FMA where the sum is too long.
+// One chunk only: k <= kChunkK.
+// Whole call, against the paired engine (us): 3500 x 3500 x 4200  1892 / 2738
+// (the slicing, now on the integer pipes, is 135 us less of each),
+// 8192^3 16660 / 22030, 1000^3 131 / 199, 250 x 300 x 400  65 / 170.  A tile of
+// k = 4200 takes 103 us of MMAs (the rate's floor is 92) and 12 us to fold; with
+// the descriptors computed in a rolled loop the issuing thread needed 160 us,
+// and an epilogue of FP64 folds with C read between the stores 48 us.
+constexpr int kRN = 48;
+constexpr int kRMaxSlices = kDefaultSlices;
+constexpr int kRRowBytes = 64;
+constexpr int kRStages = 2;
+constexpr uint32_t kRATile = BM * kRRowBytes, kRBTile = kRN * kRRowBytes;
+constexpr uint32_t kRStageBytes = kRMaxSlices * (kRATile + kRBTile);
+constexpr int kRThreads = 320;                      // TMA, MMA, 8 epilogue warps
+constexpr size_t kRSmemBytes = 1024 + kRStages * kRStageBytes + 256;
+static_assert(kRSmemBytes <= 232448, "shared memory budget");
+static_assert(kRMaxSlices * kRN <= 512, "the sums fit in tensor memory");
+
+__device__ __forceinline__ void umma_cols(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+                                          uint32_t n, uint32_t accumulate) {
+  const uint32_t idesc =
+      (1u << 4) | ((n >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+template <int S>
+__global__ void __launch_bounds__(kRThreads, 1)
+ozaki_tc_resident_kernel(const uint8_t* As, const uint8_t* Bt, TcArgs g) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + kRStages * kRStageBytes);
+  uint64_t* empty = full + kRStages;
+  uint64_t* done = empty + kRStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int st = 0; st < kRStages; ++st) {
+      mbar_init(full + st, 1);
+      mbar_init(empty + st, 1);
+    }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    mbar_init_fence();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_slot)),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  const int blocks = static_cast<int>(g.Kp / kRRowBytes);
+  const int64_t i0 = static_cast<int64_t>(raster_tile(true)) * BM;
+  const int64_t j0 = static_cast<int64_t>(raster_tile(false)) * kRN;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // columns past Np keep what shared memory held: sums that are not written
+      const uint32_t b_bytes =
+          static_cast<uint32_t>(g.Np - j0 < kRN ? g.Np - j0 : kRN) * kRRowBytes;
+      uint32_t it = 0;
+      bool ok = true;
+      for (; ok && it < static_cast<uint32_t>(blocks); ++it) {
+        const uint32_t st = it % kRStages;
+        if (!mbar_wait(empty + st, ((it / kRStages) & 1u) ^ 1u, abort_flag, g.limit_ns)) {
+          ok = false;
+          break;
+        }
+        unsigned char* a = ring + st * kRStageBytes;
+        unsigned char* b = a + kRMaxSlices * kRATile;
+        mbar_arrive_expect_tx(full + st, S * (kRATile + b_bytes));
+        const int64_t slice = static_cast<int64_t>(it) * S;
+        for (int s = 0; s < S; ++s) {
+          bulk_load(a + s * kRATile, As + ((slice + s) * g.Mp + i0) * kRRowBytes, kRATile,
+                    full + st);
+          bulk_load(b + s * kRBTile, Bt + ((slice + s) * g.Np + j0) * kRRowBytes, b_bytes,
+                    full + st);
+        }
+      }
+      if (!ok) {
+        // wind-down: let the copies already issued land before the CTA exits
+        const uint32_t first = it > static_cast<uint32_t>(kRStages) ? it - kRStages : 0u;
+        for (uint32_t j = first; j < it; ++j)
+          mbar_wait_drain(full + (j % kRStages), (j / kRStages) & 1u, g.limit_ns);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      bool ok = true;
+      for (int t = 0; ok && t < blocks; ++t) {
+        const uint32_t st = static_cast<uint32_t>(t) % kRStages;
+        if (!mbar_wait(full + st, (t / kRStages) & 1u, abort_flag, g.limit_ns)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t a_addr = smem_u32(ring + st * kRStageBytes);
+        const uint32_t b_addr = a_addr + kRMaxSlices * kRATile;
+        const uint64_t a0 = sw64_desc(a_addr), b0 = sw64_desc(b_addr);
+#pragma unroll
+        for (uint32_t kk = 0; kk < kRRowBytes / 32; ++kk) {
+#pragma unroll
+          for (int s = 0; s < S; ++s) {
+            // advance 32 bytes along K inside the swizzle atom; the first
+            // slice of A meets every weight and clears its sums
+            const uint64_t ad = a0 + (s * kRATile >> 4) + 2u * kk;
+            const uint32_t accumulate = (kk == 0 && s == 0) ? (t == 0 ? 0u : 1u) : 1u;
+#pragma unroll
+            for (int u = 0; u < S - s; u += 5) {
+              const uint32_t n = kRN * (S - s - u < 5 ? S - s - u : 5);
+              umma_cols(tmem + kRN * (s + u), ad, b0 + (u * kRBTile >> 4) + 2u * kk, n,
+                        accumulate);
+            }
+          }
+        }
+        umma_commit(empty + st);
+      }
+      // every MMA issued by this thread completes before teardown
+      umma_commit(done);
+      if (!mbar_wait_drain(done, 0u, g.limit_ns)) *abort_flag = 1;
+    }
+  } else {
+    // epilogue warps 2..9: TMEM lane quadrant warp % 4, two warps per quadrant
+    const int q = warp & 3;
+    const uint32_t col0 = kRN / 2 * static_cast<uint32_t>((warp - 2) >> 2);
+    const uint32_t at = tmem + (static_cast<uint32_t>(32 * q) << 16) + col0;
+    constexpr int kOwn = kRN / 2;  // columns per thread
+    const int64_t i = i0 + 32 * q + lane;
+    const bool row_ok = i < g.M;
+    // C is read while the MMAs run (element by element, between the stores,
+    // the reads were a chain of round trips)
+    double* row = g.C + i * g.N + j0 + col0;
+    const int own = static_cast<int>(
+        g.N - j0 - col0 < kOwn ? (g.N - j0 - col0 < 0 ? 0 : g.N - j0 - col0) : kOwn);
+    const int cols = row_ok ? own : 0;
+    double old[kOwn];
+#pragma unroll
+    for (int c = 0; c < kOwn; ++c) old[c] = (g.beta != 0.0 && c < cols) ? row[c] : 0.0;
+    const int ea = row_ok ? g.Ea[i] : 0;
+    if (mbar_wait(done, 0u, abort_flag, g.limit_ns) && __all_sync(0xffffffffu, !*abort_flag)) {
+      tc_fence_after();
+      constexpr int kLast = S + 1 < 10 ? S + 1 : 10;  // the last weight always folded as an integer
+#pragma unroll
+      for (int c = 0; c < kOwn; c += 8) {
+        int64_t sum[8];
+        uint32_t f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sum[e] = 0;
+#pragma unroll
+        for (int w = 2; w <= S + 1; ++w) {
+          tmem_ld8(at + kRN * (w - 2) + c, f);
+          tmem_ld_wait8(f);
+          if (w <= kLast) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              sum[e] = (sum[e] << kSliceBits) + __float2int_rn(__uint_as_float(f[e]));
+              if (w > 8) sum[e] = f64fix::round53(sum[e]);
+            }
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          if (c + e < cols) {
+            const int scale = ea + g.Eb[j0 + col0 + c + e];
+            const uint32_t low = static_cast<uint32_t>(1075 + scale - kSliceBits * (S + 1));
+            const bool fits = sum[e] < (1ll << 57) && sum[e] > -(1ll << 57);
+            double ab;
+            if ((kLast == S + 1 || fits) && low - 200u < 1600u) {
+              int64_t all = sum[e];
+              if (kLast < S + 1)
+                all = (all << kSliceBits) + __float2int_rn(__uint_as_float(f[e]));
+              ab = f64fix::pack(all, f64fix::Unit{low}, 0);
+            } else {
+              ab = static_cast<double>(sum[e]) * scalbn(1.0, -kSliceBits * kLast);
+              if (kLast < S + 1)
+                ab = fma(static_cast<double>(__uint_as_float(f[e])),
+                         scalbn(1.0, -kSliceBits * (S + 1)), ab);
+              ab = scalbn(ab, scale);
+            }
+            // contracted as the compiler contracts the other engines' epilogue
+            row[c + e] = (g.beta == 0.0) ? g.alpha * ab : fma(g.alpha, ab, g.beta * old[c + e]);
+          }
+        }
+      }
+    }
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag) atomicExch(g.error, 1u);
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(kTmemCols)
+                 : "memory");
+  }
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static std::once_flag once;
@@ -1046,7 +1361,7 @@ int slices_of(const b200_tune* t) {
   return (t && t->items) ? t->items : kDefaultSlices;
 }
 
-template <typename T>
+template <typename T, bool BLOCKED = false>
 int launch_slicing(const double* A, const double* B, int64_t m, int64_t n, int64_t k,
                    const SplitLayout& L, int S, char* w, cudaStream_t st) {
   int* Ea = reinterpret_cast<int*>(w + L.off_ea);
@@ -1062,11 +1377,11 @@ int launch_slicing(const double* A, const double* B, int64_t m, int64_t n, int64
   col_max_kernel<<<dim3(static_cast<unsigned>(ceil_div(n, 32)),
                         static_cast<unsigned>(k > 0 ? ceil_div(k, kColRows) : 1)),
                    dim3(32, 8), 0, st>>>(B, k, n, bmax);
-  slice_a_kernel<T><<<dim3(static_cast<unsigned>(ceil_div(L.Kp, 128 * kPer)),
+  slice_a_kernel<T, BLOCKED><<<dim3(static_cast<unsigned>(ceil_div(L.Kp, 128 * kPer)),
                            static_cast<unsigned>(L.Mp)),
                       128, 0, st>>>(A, m, k, Ea, S, L.Mp, L.Kp,
                                     reinterpret_cast<T*>(w + L.off_as));
-  slice_b_kernel<T><<<dim3(static_cast<unsigned>(L.Np / kBtJ), static_cast<unsigned>(L.Kp / kBtK)),
+  slice_b_kernel<T, BLOCKED><<<dim3(static_cast<unsigned>(L.Np / kBtJ), static_cast<unsigned>(L.Kp / kBtK)),
                       256, 0, st>>>(B, k, n, bmax, Eb, S, L.Np, L.Kp,
                                     reinterpret_cast<T*>(w + L.off_bt));
   return B200_OK;
@@ -1107,6 +1422,22 @@ int b200_gemm_split(const double* A, const double* B, double* C, int64_t m, int6
   int* Eb = reinterpret_cast<int*>(w + L.off_eb);
   cudaStream_t st = as_stream(stream);
   const bool f8 = engine == kEngineTcE4m3 || engine == kEngineTcE4m3Paired;
+  // the default takes the resident engine where its sums fit
+  if (!(tune && tune->algo) && S == kDefaultSlices && k <= kChunkK && aligned16(w)) {
+    int rc = launch_slicing<uint8_t, true>(A, B, m, n, k, L, S, w, st);
+    if (rc != B200_OK) return rc;
+    rc = allow_dynamic_smem(reinterpret_cast<const void*>(tc::ozaki_tc_resident_kernel<kDefaultSlices>),
+                            tc::kRSmemBytes, "b200_gemm_split");
+    if (rc != B200_OK) return rc;
+    const tc::TcArgs g{Ea, Eb, C, err, m, n, L.Mp, L.Np, L.Kp, alpha, beta, S,
+                       wait_limit_ns(tune, tc::kWaitLimitNs)};
+    const dim3 grid(static_cast<unsigned>(ceil_div(n, tc::kRN)),
+                    static_cast<unsigned>(L.Mp / tc::BM));
+    tc::ozaki_tc_resident_kernel<kDefaultSlices><<<grid, tc::kRThreads, tc::kRSmemBytes, st>>>(
+        reinterpret_cast<const uint8_t*>(w + L.off_as),
+        reinterpret_cast<const uint8_t*>(w + L.off_bt), g);
+    return after_launch("b200_gemm_split", 5);
+  }
   // zero-sized k: C = beta*C through the same epilogue (all digits zero)
   const int rc = f8 ? launch_slicing<uint8_t>(A, B, m, n, k, L, S, w, st)
                     : launch_slicing<__nv_bfloat16>(A, B, m, n, k, L, S, w, st);
