@@ -169,30 +169,27 @@ scan_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t n, T init,
 
 }
 
-// ---- pipelined persistent SCAN ---------------------------------------------
-// One CTA per SM on the stage ring of b200_pipeline.cuh (producer warp 0,
-// lookback warps 2-3), plus:
+// ---- pipelined persistent SCAN, int64 -----------------------------------------
+// One CTA per SM, but the scanner's, on the stage ring of b200_pipeline.cuh
+// (producer warp 0, prefix warp 2), plus:
 //  * aggregator (warp 1): sums each tile as it lands and publishes the
 //    aggregate at once;
-//  * compute (warps 4-7): a thread owns a run of 32 consecutive items (16
+//  * compute (warps 3-6): a thread owns a run of 32 consecutive items (16
 //    item pairs), sums it, scans the run sums across the tile and, when the
 //    tile's exclusive prefix arrives, writes every item's prefix in place;
-//  * store (warp 8): writes a finished tile back with one bulk store and
+//  * store (warp 7): writes a finished tile back with one bulk store and
 //    frees the stage once the store has read it (mbarrier ready[s]: compute
 //    -> store).
 // A compute thread visits its pairs rotated by (run mod 16), so every 16-byte
 // shared-memory access of a warp is conflict-free without padding the
-// bulk-copied tile.  Measured on GB300 (int64, 2^26 items, time marks per
-// tile and role): the bare load -> store pipeline runs at the copy peak; what
-// the lookback adds is its L2 round trips under saturated HBM, which the
-// seven stages of loads in flight are there to cover.
+// bulk-copied tile.
 namespace pipe {
 
 using ring::kStages;
 using ring::kTile;
 using ring::kEnd;
 constexpr int kComputeWarps = 4;
-constexpr int kFirstCompute = 2 + ring::kLookbackWarps;
+constexpr int kFirstCompute = 3;
 constexpr int kStoreWarp = kFirstCompute + kComputeWarps;
 constexpr int kThreads = 32 * (kStoreWarp + 1);
 constexpr int kRuns = 32 * kComputeWarps;    // 128 runs per tile
@@ -205,6 +202,7 @@ struct Smem {
   uint64_t ready[kStages];  // compute -> store warp: the stage holds results
   int fail_loaded;          // compute group: a wait before its first barrier gave up
   int fail_prefix;          // compute group: a wait before its second barrier gave up
+  unsigned long long ticket;  // the CTA's first
 };
 
 template <typename T>
@@ -213,9 +211,8 @@ static_assert(sizeof(Smem<long long>) + 128 <= 232448, "shared memory budget");
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
-scan_pipelined(const T* __restrict__ x, T* __restrict__ y, int64_t n, T init,
-               unsigned int tiles, ScanHeader* __restrict__ hdr,
-               TileDesc* __restrict__ descs, uint64_t limit_ns) {
+scan_pipelined(const T* x, T* y, int64_t n, T init, unsigned int tiles, ScanHeader* hdr,
+               TileDesc* descs, uint64_t limit_ns) {
   using V2 = typename Vec2<T>::type;
   extern __shared__ unsigned char s_raw[];
   Smem<T>& sm = *reinterpret_cast<Smem<T>*>(
@@ -230,10 +227,22 @@ scan_pipelined(const T* __restrict__ x, T* __restrict__ y, int64_t n, T init,
     sm.fail_prefix = 0;
     mbar_init_fence();
   }
+  const unsigned int z = begin();
+  x += z;
+  hdr += z;
+  descs += z;
+  if (tid == 0) ring::first_ticket(hdr, tiles, &sm.ticket);
   __syncthreads();
+  // the CTA with the first ticket scans the aggregates of all the others (a
+  // single tile needs no scanner)
+  const unsigned int bias = tiles > 1u ? 1u : 0u;
+  if (static_cast<unsigned int>(sm.ticket) < bias) {
+    if (warp == 0) ring::scan_aggregates(descs, tiles, init, sm.ticket >> 32, hdr, limit_ns);
+    return;
+  }
 
   if (warp == 0) {
-    ring::produce(r, x, n, tiles, hdr);
+    ring::produce(r, x, n, tiles, hdr, 1, &sm.ticket, bias);
   } else if (warp == 1) {
     // ---- aggregator: lane L sums pairs L, L + 32, ... (conflict-free) ----
     for (int k = 0;; ++k) {
@@ -251,12 +260,14 @@ scan_pipelined(const T* __restrict__ x, T* __restrict__ y, int64_t n, T init,
       }
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(0xffffffffu, total, off);
-      if (lane == 0) ring::publish_aggregate(r, descs, s, tile, total);
+      if (lane == 0) {
+        desc_store(descs + tile, r.epoch * 4 + 1, to_bits<T>(total));
+        mbar_arrive(&r.summed[s]);  // the tile is read: it may be overwritten
+      }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&r.summed[s]);
     }
   } else if (warp < kFirstCompute) {
-    ring::look_back(r, descs, init, hdr, warp - 2);
+    ring::fetch_prefixes(r, descs, init, hdr);
   } else if (warp < kStoreWarp) {
     // ---- compute ----
     // The four warps decide together whether to go on: a warp whose wait
@@ -302,7 +313,8 @@ scan_pipelined(const T* __restrict__ x, T* __restrict__ y, int64_t n, T init,
       }
       T woff = T(0);
       for (int w = 0; w < cw; ++w) woff += sm.warp_total[w];
-      const bool have_prefix = ring::wait(r, &r.prefix[s], par, hdr);
+      const bool have_prefix =
+          ring::wait(r, &r.prefix[s], par, hdr) && ring::wait(r, &r.summed[s], par, hdr);
       if (have_prefix) {
         const T base = r.excl[s] + (woff + (inc - rs));
         T run = base + head;
@@ -456,123 +468,6 @@ __device__ __forceinline__ WarpFixed warp_align(uint64_t v, uint32_t top, uint32
   return {(v + ((1ull << s) >> 1)) >> s, all - UNIT + s};
 }
 
-// The scanner: one warp, in a CTA that takes no tiles, turns the tiles'
-// aggregates, as they are published, into exclusive prefixes, in tile order.
-// Each tile's prefix warp then polls one descriptor, where a lookback re-reads
-// hundreds: at 2^26 items lookback warps in every CTA left the kernel at
-// 238-275 us (2 to 5 warps, 128 to 256 predecessors a round), the scanner at
-// 203 us (2, 4, 8 tiles per lane: 267, 203, 227 us; no prefixes at all: 173
-// us; the copy alone: 157 us).  A round takes the published tiles
-// from p on, up to kPerLane per lane.  The running prefix is kept in two parts
-// (Dekker's two-sum, larger operand first, compared as integers), so that its
-// roundings do not add up over the rounds.
-constexpr int kPerLane = 4;
-
-__device__ void scan_aggregates(TileDesc* descs, unsigned int tiles, double init,
-                                unsigned long long epoch, ScanHeader* hdr, uint64_t limit_ns) {
-  const int lane = threadIdx.x & 31;
-  const unsigned long long AGG = epoch * 4 + 1, INC = epoch * 4 + 2;
-  double hi = init, lo = 0.0;
-  uint64_t t0 = 0;  // time of the first empty round since the last full one
-  for (unsigned int p = 0; p < tiles;) {
-    double v[kPerLane];
-    unsigned int have = 0;  // the lane's published tiles before its first other one
-    {
-      unsigned long long f[kPerLane], bits[kPerLane];
-      const unsigned int t = p + lane * kPerLane;
-#pragma unroll
-      for (int j = 0; j < kPerLane; ++j) {
-        f[j] = bits[j] = 0ull;
-        if (t + j < tiles) desc_load(descs + t + j, f[j], bits[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < kPerLane; ++j) {
-        if (have == j && f[j] == AGG) ++have;
-        v[j] = have > j ? from_bits<double>(bits[j]) : 0.0;
-      }
-    }
-    const unsigned int part = __ballot_sync(0xffffffffu, have < kPerLane);
-    const int last = part ? __ffs(part) - 1 : 31;  // the last lane that counts
-    if (lane > last) have = 0;
-    const unsigned int found = last * kPerLane + __shfl_sync(0xffffffffu, have, last);
-    if (found == 0) {
-      uint64_t now = 0;
-      if (lane == 0) now = globaltimer();
-      now = __shfl_sync(0xffffffffu, now, 0);
-      if (t0 == 0) t0 = now;
-      if (now - t0 > limit_ns) {
-        if (lane == 0) atomicExch(&hdr->error, 1u);
-        return;
-      }
-      continue;
-    }
-    t0 = 0;
-    if (lane > last) {
-#pragma unroll
-      for (int j = 0; j < kPerLane; ++j) v[j] = 0.0;
-    }
-    double before[kPerLane];
-    double sum = 0.0;
-#pragma unroll
-    for (int j = 0; j < kPerLane; ++j) {
-      before[j] = sum;
-      sum += v[j];
-    }
-    const double inc = warp_inclusive_scan(sum);
-    double left = __shfl_up_sync(0xffffffffu, inc, 1);
-    left = lane == 0 ? lo : left + lo;
-#pragma unroll
-    for (int j = 0; j < kPerLane; ++j)
-      if (j < have)
-        desc_store(descs + p + lane * kPerLane + j, INC, to_bits<double>(hi + (left + before[j])));
-    const double all = __shfl_sync(0xffffffffu, inc, 31);
-    const bool first = (f64emu::bits_opaque(hi) << 1) >= (f64emu::bits_opaque(all) << 1);
-    const double a = first ? hi : all, b = first ? all : hi;
-    hi = a + b;
-    const double err = b - (hi - a);
-    lo += fabs(err) < INFINITY ? err : 0.0;
-    p += found;
-  }
-}
-
-// The prefix warp: takes each tile's exclusive prefix from the scanner.
-__device__ void fetch_prefixes(Smem& sm, const TileDesc* descs, double init, ScanHeader* hdr) {
-  auto& r = sm.r;
-  const int lane = threadIdx.x & 31;
-  for (int k = 0;; ++k) {
-    const int s = k % kStages;
-    if (!ring::wait(r, &r.drawn[s], (k / kStages) & 1, hdr)) return;
-    const unsigned int tile = r.ticket[s];
-    if (tile == kEnd) return;
-    if (lane == 0) {
-      const unsigned long long INC = r.epoch * 4 + 2;
-      double excl = init;
-      bool ok = true;
-      if (tile > 0) {
-        unsigned long long f, bits;
-        desc_load(descs + tile, f, bits);
-        if (f != INC) {
-          const uint64_t t0 = globaltimer();
-          while (ok && f != INC) {
-            desc_load(descs + tile, f, bits);
-            ok = globaltimer() - t0 <= r.limit_ns;
-          }
-        }
-        excl = from_bits<double>(bits);
-      }
-      if (ok) {
-        r.excl[s] = excl;
-        mbar_arrive(&r.prefix[s]);
-      } else {
-        atomicExch(&hdr->error, 1u);
-        *reinterpret_cast<volatile int*>(&r.abort) = 1;
-      }
-    }
-    __syncwarp();
-    if (*reinterpret_cast<volatile int*>(&r.abort)) return;
-  }
-}
-
 __global__ void __launch_bounds__(kThreads, 1)
 scan_pipelined_f64(const double* x, double* y, int64_t n, double init, unsigned int tiles,
                    ScanHeader* hdr, TileDesc* descs, uint64_t limit_ns, int zero) {
@@ -594,26 +489,20 @@ scan_pipelined_f64(const double* x, double* y, int64_t n, double init, unsigned 
   x += z;
   hdr += z;
   descs += z;
-  if (tid == 0) {
-    const unsigned long long draws = static_cast<unsigned long long>(tiles) + gridDim.x;
-    const unsigned long long t = atomicAdd(&hdr->ticket, 1ull);
-    if (static_cast<unsigned int>(t) == draws - 1)
-      atomicAdd(&hdr->ticket, (1ull << 32) - draws);
-    sm.ticket = t;
-  }
+  if (tid == 0) ring::first_ticket(hdr, tiles, &sm.ticket);
   __syncthreads();
   // the CTA with the first ticket scans the aggregates of all the others (a
   // single tile needs no scanner)
   const unsigned int bias = tiles > 1u ? 1u : 0u;
   if (static_cast<unsigned int>(sm.ticket) < bias) {
-    if (warp == 0) scan_aggregates(descs, tiles, init, sm.ticket >> 32, hdr, limit_ns);
+    if (warp == 0) ring::scan_aggregates(descs, tiles, init, sm.ticket >> 32, hdr, limit_ns);
     return;
   }
 
   if (warp == 0) {
     ring::produce(r, x, n, tiles, hdr, kGroups, &sm.ticket, bias);
   } else if (warp < kFirstAgg) {
-    fetch_prefixes(sm, descs, init, hdr);
+    ring::fetch_prefixes(r, descs, init, hdr);
   } else if (warp < kFirstCompute) {
     // ---- aggregators ----
     const int aw = warp - kFirstAgg, run = aw * 32 + lane;
@@ -827,10 +716,11 @@ int launch_scan_pipelined(const long long* x, long long* y, int64_t n, long long
       reinterpret_cast<const void*>(pipe::scan_pipelined<long long>), kSmem, "scan");
   if (rc != B200_OK) return rc;
   const int64_t tiles = ceil_div(n, pipe::kTile);
-  const int grid = static_cast<int>(std::min<int64_t>(tiles, device_info().sm_count));
-  pipe::scan_pipelined<long long><<<grid, pipe::kThreads, kSmem, st>>>(
-      x, y, n, init, static_cast<unsigned int>(tiles), reinterpret_cast<ScanHeader*>(w),
-      reinterpret_cast<TileDesc*>(w + 256), limit_ns);
+  const int grid =
+      static_cast<int>(std::min<int64_t>(tiles > 1 ? tiles + 1 : 1, device_info().sm_count));
+  launch(pipe::scan_pipelined<long long>, grid, pipe::kThreads, kSmem, st, x, y, n, init,
+         static_cast<unsigned int>(tiles), reinterpret_cast<ScanHeader*>(w),
+         reinterpret_cast<TileDesc*>(w + 256), limit_ns);
   return B200_OK;
 }
 

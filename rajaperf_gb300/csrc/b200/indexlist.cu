@@ -13,7 +13,7 @@
 // same list and count; it runs through the same single pass.
 //
 // Default (x 16-byte aligned): a persistent form on bulk copies and the
-// lookback warps of b200_pipeline.cuh (one CTA per SM).  Unlike SCAN it frees
+// scanner of b200_pipeline.cuh (one CTA per SM).  Unlike SCAN it frees
 // a tile's shared-memory stage as soon as the tile's items are ranked (their
 // selection bits are all the list needs), so the stages keep loading while
 // tiles wait for their base counts in small slots.  tune->algo = 1 (and an unaligned x) runs
@@ -23,6 +23,7 @@
 #include "b200_internal.cuh"
 #include "b200_async.cuh"
 #include "b200_f64emu.cuh"
+#include "b200_launch.cuh"
 #include "b200_lookback.cuh"
 #include "b200_pipeline.cuh"
 
@@ -134,28 +135,23 @@ int64_t tiles_of(int64_t n) { return ceil_div(n > 0 ? n : 1, kTile); }
 // have turned a tile into its selection bits (4096 bits, 512 bytes) the
 // tile's shared-memory stage is refilled, and the tile waits for its base
 // count in a small slot instead.  So the x stages stay busy loading while
-// the lookback (the wait for every predecessor's count) is covered by many
+// the wait for the base count (every predecessor's count) is covered by many
 // cheap slots: kData 32 KB stages, kSlots 512-byte slots.
 //   warp 0                  producer: draws runs of four consecutive tile ids
 //                           per atomic, one bulk copy per tile
-//   warps 1-4               lookback: one global walk per run, the run's
-//                           other base counts from its own tile counts
-//   warps 5-12 (ballot)     two groups of four on alternate tiles: rank the
+//   warp 1                  prefix: each tile's base count from the scanner
+//   warps 2-9 (ballot)      two groups of four on alternate tiles: rank the
 //                           tile's items in rows of 64 (two ballots per row),
 //                           publish the tile's count, free the stage
-//   warps 13-20 (writer)    two groups of four on alternate tiles: with the
+//   warps 10-17 (writer)    two groups of four on alternate tiles: with the
 //                           base count, write the selected indices to
 //                           consecutive list entries, free the slot
-// Measured per tile on GB300 (2^27 items, %globaltimer marks) with one
-// lookback pair and four-warp groups: load 3.1 us, ballots 0.9 us, a walk
-// 2.5 us, writes 1.3 us; two walks in flight per SM bounded the draw rate at
-// 0.7 tiles per us per SM (60% of the copy peak), the four-warp groups close
-// behind.  Each role now keeps two to four tiles in flight.
+// Measured (2^24 + 4093 items, half of them selected): 46 us with four lookback
+// warps per CTA, 44 us with the scanner (b200_pipeline.cuh).
 // Per slot b, one arrival each: drawn[b] (producer), summed[b] (ballot
-// group), prefix[b] (lookback), empty[b] (writer group); per stage d: full[d]
+// group), prefix[b] (prefix warp), empty[b] (writer group); per stage d: full[d]
 // (bulk copy), data_empty[d] (ballot group).  The ballot and writer groups
-// and the lookback warps take alternate tiles and wait on drawn[b] first (the
-// ring's rule).
+// take alternate tiles and wait on drawn[b] first (the ring's rule).
 namespace ilpipe {
 
 using ring::kEnd;
@@ -166,11 +162,9 @@ constexpr int kGroups = 2;                   // ballot groups, and writer groups
 constexpr int kGroupWarps = 4;               // warps per group
 constexpr int kSeg = kTile / kGroupWarps;    // 1024 items per warp
 constexpr int kRows = kSeg / 64;             // 16 rows of 64 items (a lane holds a pair)
-constexpr int kLookbackWarps = 4;            // runs in flight per SM
 constexpr int kDraw = 4;                     // tile ids per draw: a run
-constexpr int kEnds = kDraw * kLookbackWarps;  // end markers
-constexpr int kFirstLookback = 1;
-constexpr int kFirstBallot = kFirstLookback + kLookbackWarps;
+constexpr int kEnds = kGroups;               // end markers
+constexpr int kFirstBallot = 2;              // after the producer and the prefix warp
 constexpr int kFirstWriter = kFirstBallot + kGroups * kGroupWarps;
 constexpr int kThreads = 32 * (kFirstWriter + kGroups * kGroupWarps);
 static_assert(kGroups < kData && kGroups < kSlots, "alternate-tile groups see phases in order");
@@ -183,6 +177,7 @@ static_assert(kRows <= 32, "a lane holds one row's ballots");
 // ring::publish_aggregate).
 struct Slots {
   using AccT = long long;
+  static constexpr int kStages = kSlots;
   long long agg[kSlots];
   long long excl[kSlots];
   unsigned int ticket[kSlots];
@@ -205,14 +200,13 @@ struct Smem {
   Slots r;
   int fail_ballot[kGroups];  // per ballot group: a wait gave up
   int fail_writer[kGroups];  // per writer group: a wait gave up
+  unsigned long long ticket;  // the CTA's first
 };
 static_assert(sizeof(Smem) + 128 <= 232448, "shared memory budget");
 
 __global__ void __launch_bounds__(kThreads, 1)
-indexlist_pipelined(const double* __restrict__ x, int32_t* __restrict__ list, int64_t n,
-                    int64_t* __restrict__ len, unsigned int tiles,
-                    ScanHeader* __restrict__ hdr, TileDesc* __restrict__ descs,
-                    uint64_t limit_ns) {
+indexlist_pipelined(const double* x, int32_t* list, int64_t n, int64_t* len, unsigned int tiles,
+                    ScanHeader* hdr, TileDesc* descs, uint64_t limit_ns) {
   extern __shared__ unsigned char s_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(
       (reinterpret_cast<uintptr_t>(s_raw) + 127) & ~static_cast<uintptr_t>(127));
@@ -236,19 +230,32 @@ indexlist_pipelined(const double* __restrict__ x, int32_t* __restrict__ list, in
     for (int g = 0; g < kGroups; ++g) sm.fail_ballot[g] = sm.fail_writer[g] = 0;
     mbar_init_fence();
   }
+  const unsigned int z = begin();
+  x += z;
+  hdr += z;
+  descs += z;
+  if (tid == 0) ring::first_ticket(hdr, tiles, &sm.ticket, kDraw);
   __syncthreads();
+  // the CTA with the first ticket scans the counts of all the others (a single
+  // tile needs no scanner)
+  const unsigned int bias = tiles > 1u ? static_cast<unsigned int>(kDraw) : 0u;
+  if (static_cast<unsigned int>(sm.ticket) < bias) {
+    if (warp == 0)
+      ring::scan_aggregates<long long>(descs, tiles, 0, sm.ticket >> 32, hdr, limit_ns);
+    return;
+  }
 
   if (warp == 0) {
     // ---- producer: tile k takes slot k % kSlots and stage k % kData.  One
     // atomic draws a run of kDraw consecutive tile ids once their slots are
     // free (a round trip to the ticket counter per tile bounded the CTA's
-    // tile rate, and a run needs one global lookback, not kDraw); each tile's
-    // bulk copy is issued as soon as its stage is free.  A CTA stops at the
+    // tile rate); each tile's bulk copy is issued as soon as its stage is
+    // free.  The CTA's first draw was made at its start.  A CTA stops at the
     // first draw that reaches the end: floor(tiles / kDraw) draws stop no
-    // CTA, so the launch makes floor(tiles / kDraw) + gridDim.x draws and the
-    // CTA making the last one resets the count and advances the epoch.  Ids
-    // past the end are end markers, then more, kEnds in all, so that every
-    // lookback warp's next run starts with one; end markers take no stage.
+    // CTA, so the launch makes floor(tiles / kDraw) + gridDim.x draws, the
+    // scanner's among them, and the CTA making the last one resets the count
+    // and advances the epoch.  Ids past the end are end markers, then more,
+    // kEnds in all, so that every group meets one; end markers take no stage.
     const unsigned long long draws = tiles / kDraw + gridDim.x;
     volatile int* abort_flag = &r.abort;
     int ends = 0;
@@ -264,14 +271,16 @@ indexlist_pipelined(const double* __restrict__ x, int32_t* __restrict__ list, in
       unsigned int first = kEnd;
       if (ends == 0) {
         unsigned long long t = 0;
-        if (lane == 0) {
+        if (k == 0) {
+          t = sm.ticket;
+        } else if (lane == 0) {
           t = atomicAdd(&hdr->ticket, static_cast<unsigned long long>(kDraw));
           if (static_cast<unsigned int>(t) == kDraw * (draws - 1))
             atomicAdd(&hdr->ticket, (1ull << 32) - kDraw * draws);
         }
         t = __shfl_sync(0xffffffffu, t, 0);
         if (k == 0 && lane == 0) r.epoch = t >> 32;
-        first = static_cast<unsigned int>(t);
+        first = static_cast<unsigned int>(t) - bias;
       }
       const bool drawing = ends == 0;
       if (lane == 0)
@@ -309,44 +318,7 @@ indexlist_pipelined(const double* __restrict__ x, int32_t* __restrict__ list, in
       if (!ok) break;
     }
   } else if (warp < kFirstBallot) {
-    // ---- lookback: warp lw takes the runs q = lw, lw + W, ...  (run q = the
-    // CTA's tiles q kDraw .. q kDraw + kDraw - 1, consecutive ids).  One
-    // global walk gives the run's first tile its exclusive count; each next
-    // tile's is the previous one's plus that tile's count (no global walk).
-    // Every tile's inclusive count is published as soon as it is known.
-    const int lw = warp - kFirstLookback;
-    bool done = false;
-    for (int q = lw; !done; q += kLookbackWarps) {
-      long long excl = 0;
-      for (int i = 0; i < kDraw; ++i) {
-        const int k = q * kDraw + i, b = k % kSlots;
-        const uint32_t par = (k / kSlots) & 1;
-        if (!ring::wait(r, &r.drawn[b], par, hdr)) {
-          done = true;
-          break;
-        }
-        const unsigned int tile = r.ticket[b];
-        if (tile == kEnd) {
-          done = true;
-          break;
-        }
-        const unsigned long long AGG = r.epoch * 4 + 1, INC = r.epoch * 4 + 2;
-        if (i == 0 && tile > 0)
-          excl = lookback_exclusive<long long, ring::kLookbackLanes>(descs, tile, AGG, INC, hdr,
-                                                                     r.limit_ns);
-        if (!ring::wait(r, &r.summed[b], par, hdr)) {
-          done = true;
-          break;
-        }
-        if (lane == 0) {
-          desc_store(descs + tile, INC, to_bits<long long>(excl + r.agg[b]));
-          r.excl[b] = excl;
-        }
-        excl += r.agg[b];
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&r.prefix[b]);
-      }
-    }
+    ring::fetch_prefixes(r, descs, 0, hdr);
   } else if (warp < kFirstWriter) {
     // ---- ballot group: warp cw owns items [cw * kSeg, cw * kSeg + kSeg) of a
     // tile; row u = items 64u .. 64u + 63, lane L the pair 64u + 2L, +1
@@ -383,7 +355,8 @@ indexlist_pipelined(const double* __restrict__ x, int32_t* __restrict__ list, in
         long long total = 0;
 #pragma unroll
         for (int w = 0; w < kGroupWarps; ++w) total += sm.wcount[b][w];
-        ring::publish_aggregate(r, descs, b, tile, total);
+        r.agg[b] = total;
+        desc_store(descs + tile, r.epoch * 4 + 1, to_bits<long long>(total));
         mbar_arrive(&r.summed[b]);
       }
     }
@@ -400,7 +373,8 @@ indexlist_pipelined(const double* __restrict__ x, int32_t* __restrict__ list, in
       const uint32_t par = (k / kSlots) & 1;
       bool ok = ring::wait(r, &r.drawn[b], par, hdr);
       const unsigned int tile = ok ? r.ticket[b] : kEnd;
-      if (ok && tile != kEnd) ok = ring::wait(r, &r.prefix[b], par, hdr);
+      if (ok && tile != kEnd)
+        ok = ring::wait(r, &r.prefix[b], par, hdr) && ring::wait(r, &r.summed[b], par, hdr);
       if (!ok) *fail = 1;
       if (ok && tile != kEnd) {
         long long off = r.excl[b];
@@ -479,9 +453,10 @@ int b200_basic_indexlist(const double* x, int32_t* list, int64_t n, int64_t* len
                                       kSmem, "b200_basic_indexlist");
     if (rc != B200_OK) return rc;
     const int64_t tiles = ceil_div(n, ilpipe::kTile);
-    const int grid = static_cast<int>(std::min<int64_t>(tiles, device_info().sm_count));
-    ilpipe::indexlist_pipelined<<<grid, ilpipe::kThreads, kSmem, st>>>(
-        x, list, n, len, static_cast<unsigned int>(tiles), hdr, descs, lim);
+    const int grid =
+        static_cast<int>(std::min<int64_t>(tiles > 1 ? tiles + 1 : 1, device_info().sm_count));
+    launch(ilpipe::indexlist_pipelined, grid, ilpipe::kThreads, kSmem, st, x, list, n, len,
+           static_cast<unsigned int>(tiles), hdr, descs, lim);
     return after_launch("b200_basic_indexlist");
   }
   const unsigned tiles = static_cast<unsigned>(tiles_of(n));
