@@ -4,6 +4,7 @@
 // macro's operation order.
 #include "b200_internal.cuh"
 #include "b200_f64emu.cuh"
+#include "b200_f64fix.cuh"
 #include "b200_fma_form.cuh"
 #include "b200_map.cuh"
 #include "b200_reduce.cuh"
@@ -311,12 +312,17 @@ hydro2d_body1(double* za, double* zb, const double* zm, const double* zp, const 
 // FP64 pipe after the loop; a thread holds at most 64 points (the launcher
 // checks), one bit each.  An FP64 redo inside the loop would be compiled as
 // predicated FP64 instructions, which occupy the FP64 pipe in every warp.
+// KH = kHydroFixed, the default: all eight differences in fixed point (f64fix),
+// the point's own value unpacked once for four of them: 12 FP64 instructions a
+// point instead of 14, and fewer integer ones (the rep at 1999 x 2003: 187 -> 174
+// us).
+constexpr int kHydroFixed = 9;
 template <int BS, int KH>
 __global__ void __launch_bounds__(BS)
 hydro2d_body23(const double* za, const double* zb, const double* zr, double* zu, double* zv,
                const double* zz, double* zrout, double* zzout, double s, double t, int64_t kn,
                int64_t jn, int zero) {
-  static_assert(KH >= 0 && KH <= 8, "0..8 integer-pipe differences");
+  static_assert(KH >= 0 && KH <= kHydroFixed, "0..8 integer-pipe differences, or all fixed-point");
   const int64_t j = 1 + begin() + static_cast<int64_t>(blockIdx.x) * BS + threadIdx.x;
   if (j >= jn - 1) return;
   const unsigned live = __activemask();
@@ -334,12 +340,23 @@ hydro2d_body23(const double* za, const double* zb, const double* zr, double* zu,
     const double zz0 = ld(zz + c), zr0 = ld(zr + c);
     const int64_t off[4] = {1, -1, -jn, jn};
     double du[4], dv[4];
+    if (KH == kHydroFixed && use_int) {
+      const f64fix::Unit uz = f64fix::unit_at(zz0, 3, slow), ur = f64fix::unit_at(zr0, 3, slow);
+      const int64_t fz = f64fix::fix(zz0, uz, slow), fr0 = f64fix::fix(zr0, ur, slow);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const double zn = ld(zz + c + off[m]), rn = ld(zr + c + off[m]);
-      du[m] = (use_int && m < KH) ? f64emu::sub_near_fast(zz0, zn, slow) : fform::sub(zz0, zn, fr);
-      dv[m] = (use_int && m + 4 < KH) ? f64emu::sub_near_fast(zr0, rn, slow)
-                                      : fform::sub(zr0, rn, fr);
+      for (int m = 0; m < 4; ++m) {
+        du[m] = f64fix::pack(fz - f64fix::fix(ld(zz + c + off[m]), uz, slow), uz, 0);
+        dv[m] = f64fix::pack(fr0 - f64fix::fix(ld(zr + c + off[m]), ur, slow), ur, 0);
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const double zn = ld(zz + c + off[m]), rn = ld(zr + c + off[m]);
+        du[m] = (use_int && m < KH) ? f64emu::sub_near_fast(zz0, zn, slow)
+                                    : fform::sub(zz0, zn, fr);
+        dv[m] = (use_int && m + 4 < KH) ? f64emu::sub_near_fast(zr0, rn, slow)
+                                        : fform::sub(zr0, rn, fr);
+      }
     }
     // zu + s * (((za0 du1 - za1 du2) - zb0 du3) + zb1 du4), left to right as
     // the suite writes it, the products after the first and s * (...) as FMAs
@@ -559,13 +576,11 @@ int b200_lcals_planckian(const double* x, double* y, const double* u, const doub
                       as_stream(stream));
 }
 
-// HYDRO_2D's BODY2 differences on the integer pipes by default (of 8).
+// HYDRO_2D's BODY2 differences on the integer pipes one by one (tune->tile_z).
 // Measured on GB300 (us per rep at 4096^2, BODY1 + BODY2/3, 64 threads):
 // 0: 864.9, 2: 815.1, 4: 764.5, 6: 756.4, 8: 832.1 (BODY2/3 alone: 546 us
 // at 0, 447 at 4 with the FP64 pipe 97% and the integer ALU 55% busy, 516
 // at 8 with the ALU 90% busy and the FP64 pipe 63%).
-constexpr int kHydroIntSubs = 6;
-
 int b200_lcals_hydro_2d(double* za, double* zb, const double* zm, const double* zp,
                         const double* zq, const double* zr, double* zu, double* zv,
                         const double* zz, double* zrout, double* zzout, double s,
@@ -581,8 +596,8 @@ int b200_lcals_hydro_2d(double* za, double* zb, const double* zm, const double* 
   dim3 grid = rows_grid(jn, kn, bs);
   // tune->tile_z = 1 + differences of BODY2 on the integer pipes (0, 2, 4,
   // 6 or 8); 0 keeps the default
-  int kh = (tune && tune->tile_z > 0) ? tune->tile_z - 1 : kHydroIntSubs;
-  if (kh < 0 || kh > 8 || (kh & 1)) return invalid("b200_lcals_hydro_2d: bad tile_z");
+  int kh = (tune && tune->tile_z > 0) ? tune->tile_z - 1 : kHydroFixed;
+  if (tune && tune->tile_z > 0 && (kh > 8 || (kh & 1))) return invalid("b200_lcals_hydro_2d: bad tile_z");
   if (ceil_div(kn - 2, static_cast<int64_t>(grid.y)) > 64) kh = 0;  // one redo bit per point
   B200_DISPATCH_BLOCK(bs, BS,
     launch(hydro2d_body1<BS>, grid, BS, 0, st, za, zb, zm, zp, zq, zr, kn, jn, 0);
@@ -595,7 +610,8 @@ int b200_lcals_hydro_2d(double* za, double* zb, const double* zm, const double* 
       case 2: body23(std::integral_constant<int, 2>{}); break;
       case 4: body23(std::integral_constant<int, 4>{}); break;
       case 6: body23(std::integral_constant<int, 6>{}); break;
-      default: body23(std::integral_constant<int, 8>{}); break;
+      case 8: body23(std::integral_constant<int, 8>{}); break;
+      default: body23(std::integral_constant<int, kHydroFixed>{}); break;
     });
   return after_launch("b200_lcals_hydro_2d", 2);
 }
