@@ -216,9 +216,9 @@ def _bandwidth_cases():
                                   8 * 6 * (kn - 2) * (jn - 2))
             self.flops_per_rep = 44 * (kn - 2) * (jn - 2)
             # ncu: BODY1 10 per point (its divisions and products run on the
-            # integer and FP32 pipes), BODY2+BODY3 14 per point (6 of its 8
+            # integer and FP32 pipes), BODY2+BODY3 12 per point (its 8
             # differences on the integer pipes)
-            self.fp64_instr_per_rep = 24 * (kn - 2) * (jn - 2)
+            self.fp64_instr_per_rep = 22 * (kn - 2) * (jn - 2)
 
         def run(self, s):
             a = [t.data_ptr() for t in self.arr]
@@ -295,10 +295,10 @@ def _bandwidth_cases():
             self.div = self.zeros(nn)
             self.bytes_per_rep = 8 * self.nz + 4 * 8 * n_real_nodes + 8 * self.nz
             self.flops_per_rep = 54 * self.nz
-            # 27 per zone: of the 30 adds and 3 FMAs, the first add of six
-            # corner sums runs on the integer pipes, as do the halves,
-            # divisions, standalone products and + ptiny
-            self.fp64_instr_per_rep = 27 * self.nz
+            # 19 per zone: of the 30 adds and 3 FMAs, the coordinate sums run
+            # on the integer pipes, as do the halves, divisions, standalone
+            # products and + ptiny
+            self.fp64_instr_per_rep = 19 * self.nz
 
         def run(self, s):
             return self.L.b200_apps_del_dot_vec_2d(
@@ -317,9 +317,9 @@ def _bandwidth_cases():
             self.A, self.B = self.uniform(N * N), self.uniform(N * N)
             self.bytes_per_rep = (8 * (N * N - 4) * 2 + 8 * (N - 2) * (N - 2) * 2) * tsteps
             self.flops_per_rep = tsteps * 10 * (N - 2) * (N - 2)
-            # per point and half-step: three of the four adds on the FP64 pipe
-            # (the first add and the product by 0.2 run on the integer pipes)
-            self.fp64_instr_per_rep = tsteps * 6 * (N - 2) * (N - 2)
+            # per point and half-step: two of the four adds on the FP64 pipe
+            # (the last two and the product by 0.2 run on the integer pipes)
+            self.fp64_instr_per_rep = tsteps * 4 * (N - 2) * (N - 2)
 
         def run(self, s):
             return self.L.b200_polybench_jacobi_2d(self.A.data_ptr(), self.B.data_ptr(), self.N,
@@ -337,9 +337,9 @@ def _bandwidth_cases():
             inner = (N - 2) ** 3
             self.bytes_per_rep = (8 * (N ** 3 - 12 * (N - 2) - 8) * 2 + 8 * inner * 2) * tsteps
             self.flops_per_rep = tsteps * 30 * inner
-            # per point and half-step: 9 adds, 2.5 of them (5 of the 6
-            # differences b(+1) - 2a of two planes) on the integer pipes
-            self.fp64_instr_per_rep = tsteps * 13 * inner
+            # per point and half-step: 4 in three rows of four, 1 in the fourth
+            # (the rest of its adds run on the integer pipes)
+            self.fp64_instr_per_rep = tsteps * 6.5 * inner
 
         def run(self, s):
             return self.L.b200_polybench_heat_3d(self.A.data_ptr(), self.B.data_ptr(), self.N,

@@ -57,9 +57,9 @@ struct Eos {
 };
 
 // Element map with part of each element's FP64 work on the integer pipes.
-// F::split(i, regs, slow) computes element i with some operations in an
+// F::load(i) reads element i, F::split(in, regs, slow) computes it with some operations in an
 // exact integer form (bit-identical to the FP64 pipe's) and sets `slow` when
-// an operand leaves that form's range; F::exact(i, regs) is the all-FP64
+// an operand leaves that form's range; F::exact(in, regs) is the all-FP64
 // form.  A CTA covers PT * BS consecutive elements, a thread every BS-th of
 // them (coalesced).  An element that met `slow` stores nothing in the loop
 // and is redone with F::exact after it (one bit per element): an FP64 redo
@@ -71,34 +71,33 @@ __global__ void __launch_bounds__(BS) split_map_kernel(F f, int64_t n) {
   const int64_t base = static_cast<int64_t>(blockIdx.x) * BS * PT + threadIdx.x + begin();
   const auto rg = f.regs();
   uint64_t redo = 0;
-  double v[PT];
+  typename F::In in[PT];
   auto element = [&](int p) {
     bool slow = false;
-    v[p] = f.split(base + static_cast<int64_t>(p) * BS, rg, slow);
-    if (slow) redo |= 1ull << p;
-  };
-  auto store = [&](int p) {
-    if (!((redo >> p) & 1u)) f.store(base + static_cast<int64_t>(p) * BS, v[p]);
+    const double v = f.split(in[p], rg, slow);
+    if (!slow) f.store(base + static_cast<int64_t>(p) * BS, v);
+    else redo |= 1ull << p;
   };
   if (static_cast<int64_t>(blockIdx.x + 1) * BS * PT <= n) {
     // a whole CTA in range: no bounds test, so the unrolled elements' loads
-    // issue together
+    // issue together, before the first store
+#pragma unroll
+    for (int p = 0; p < PT; ++p) in[p] = f.load(base + static_cast<int64_t>(p) * BS);
 #pragma unroll
     for (int p = 0; p < PT; ++p) element(p);
-#pragma unroll
-    for (int p = 0; p < PT; ++p) store(p);
   } else {
 #pragma unroll
     for (int p = 0; p < PT; ++p)
-      if (base + static_cast<int64_t>(p) * BS < n) element(p);
+      if (base + static_cast<int64_t>(p) * BS < n)
+        in[p] = f.load(base + static_cast<int64_t>(p) * BS);
 #pragma unroll
     for (int p = 0; p < PT; ++p)
-      if (base + static_cast<int64_t>(p) * BS < n) store(p);
+      if (base + static_cast<int64_t>(p) * BS < n) element(p);
   }
   if (__any_sync(__activemask(), redo != 0)) {
     for (int p = 0; p < PT; ++p) {
       const int64_t i = base + static_cast<int64_t>(p) * BS;
-      if (i < n && ((redo >> p) & 1u)) f.store(i, f.exact(i, rg));
+      if (i < n && ((redo >> p) & 1u)) f.store(i, f.exact(f.load(i), rg));
     }
   }
 }
@@ -118,22 +117,29 @@ struct EosSplit {
   __device__ Regs regs() const {
     return {fform::reg(q, zero), fform::reg(r, zero), fform::reg(t, zero)};
   }
-  __device__ double split(int64_t i, const Regs& g, bool& slow) const {
+  struct In { double y, z, u[7]; };
+  __device__ In load(int64_t i) const {
+    In e{ld(y + i), ld(z + i), {}};
+#pragma unroll
+    for (int k = 0; k < 7; ++k) e.u[k] = ld(u + i + k);
+    return e;
+  }
+  __device__ double split(const In& e, const Regs& g, bool& slow) const {
     auto f = [&](int m, double a, double b, double c) {
       return (m < KF) ? f64emu::fma_pos_fast(a, b, c, slow) : fma(a, b, c);
     };
-    const double a1 = f(0, g.r, ld(y + i), ld(z + i));
-    const double b1 = f(1, g.r, ld(u + i + 1), ld(u + i + 2));
-    const double c1 = f(2, g.q, ld(u + i + 4), ld(u + i + 5));
-    const double a = f(3, g.r, a1, ld(u + i));
-    const double b = f(4, g.r, b1, ld(u + i + 3));
-    const double c = f(5, g.q, c1, ld(u + i + 6));
+    const double a1 = f(0, g.r, e.y, e.z);
+    const double b1 = f(1, g.r, e.u[1], e.u[2]);
+    const double c1 = f(2, g.q, e.u[4], e.u[5]);
+    const double a = f(3, g.r, a1, e.u[0]);
+    const double b = f(4, g.r, b1, e.u[3]);
+    const double c = f(5, g.q, c1, e.u[6]);
     return f(7, g.t, f(6, g.t, c, b), a);
   }
-  __device__ double exact(int64_t i, const Regs& g) const {
-    const double a = fma(g.r, fma(g.r, ld(y + i), ld(z + i)), ld(u + i));
-    const double b = fma(g.r, fma(g.r, ld(u + i + 1), ld(u + i + 2)), ld(u + i + 3));
-    const double c = fma(g.q, fma(g.q, ld(u + i + 4), ld(u + i + 5)), ld(u + i + 6));
+  __device__ double exact(const In& e, const Regs& g) const {
+    const double a = fma(g.r, fma(g.r, e.y, e.z), e.u[0]);
+    const double b = fma(g.r, fma(g.r, e.u[1], e.u[2]), e.u[3]);
+    const double c = fma(g.q, fma(g.q, e.u[4], e.u[5]), e.u[6]);
     return fma(g.t, fma(g.t, c, b), a);
   }
   __device__ void store(int64_t i, double v) const { x[i] = v; }
