@@ -245,8 +245,9 @@ int b200_lcals_hydro_1d(double* x, const double* y, const double* z, double q,
 /* One rep of HYDRO_2D on a kn x jn row-major grid (index j + k*jn): BODY1
  * (za, zb) then BODY2 (zu, zv +=) and BODY3 (zrout, zzout) over the interior
  *   -- lcals/HYDRO_2D.hpp:66-90, HYDRO_2D-Cuda.cpp:104-140.  Two launches.
- * tune->tile_z - 1 of BODY2's eight differences (0, 2, 4, 6, 8; default 6)
- * run on the integer pipes (exact, bit-identical).                          */
+ * BODY2's eight differences run on the integer pipes in fixed point (exact,
+ * bit-identical); tune->tile_z - 1 of them (0, 2, 4, 6 or 8) one by one
+ * instead.                                                                  */
 int b200_lcals_hydro_2d(double* za, double* zb, const double* zm,
                         const double* zp, const double* zq, const double* zr,
                         double* zu, double* zv, const double* zz, double* zrout,
@@ -326,10 +327,10 @@ int b200_apps_vol3d(const double* x, const double* y, const double* z,
 /* Nodal divergence for each real zone i = real_zones[ii], corners i, i+1,
  * i+1+jp, i+jp  -- apps/DEL_DOT_VEC_2D.hpp:65-90, DEL_DOT_VEC_2D-Cuda.cpp:30-60
  * With half = 0.5 the halvings are exponent moves, the divisions and five
- * products integer-pipe arithmetic and the first add of six of the eight
- * corner sums integer-pipe adds, all bit-identical to the FP64 pipe;
- * tune->tile_z = 1 + corner sums opened on the integer pipes (0, 2, 4, 6 or 8;
- * default 6). */
+ * products integer-pipe arithmetic and the sums over x and y fixed-point
+ * integer adds, all bit-identical to the FP64 pipe; tune->tile_z = 1 + corner
+ * sums whose first add alone runs on the integer pipes (0, 2, 4, 6 or 8)
+ * instead. */
 int b200_apps_del_dot_vec_2d(const double* x, const double* y,
                              const double* xdot, const double* ydot,
                              double* div, const int64_t* real_zones,

@@ -1100,10 +1100,18 @@ int b200_polybench_3mm(const double* A, const double* B, const double* C,
   // tune->algo 1: the FP64 pipe
   if (!(tune && tune->algo == 1) && dgemm_tc_takes(p[0]) && dgemm_tc_takes(p[1]) &&
       dgemm_tc_takes(p[2])) {
-    int s = launch_dgemm_tc(p, 2, st);
+    // E and F in one launch, unless one is written where the other's operands lie
+    auto apart = [](const double* a, int64_t an, const double* b, int64_t bn) {
+      return a + an <= b || b + bn <= a;
+    };
+    const bool together = apart(E, ni * nj, C, nj * nm) && apart(E, ni * nj, D, nm * nl) &&
+                          apart(F, nj * nl, A, ni * nk) && apart(F, nj * nl, B, nk * nj) &&
+                          apart(E, ni * nj, F, nj * nl);
+    int s = launch_dgemm_tc(p, together ? 2 : 1, st);
+    if (s == B200_OK && !together) s = launch_dgemm_tc(p + 1, 1, st);
     if (s == B200_OK) s = launch_dgemm_tc(p + 2, 1, st);
     if (s != B200_OK) return s;
-    return after_launch("b200_polybench_3mm", 2);
+    return after_launch("b200_polybench_3mm", together ? 2 : 3);
   }
   int s = launch_dgemm(A, B, E, ni, nj, nk, 1.0, 0.0, 0, st);   // E = A*B
   if (s == B200_OK) s = launch_dgemm(C, D, F, nj, nl, nm, 1.0, 0.0, 0, st);  // F = C*D

@@ -106,3 +106,20 @@ def test_more_accurate_than_the_fp64_pipe():
     err = [float(np.linalg.norm((_mm3(mats, dims, t)[0] - want).astype(np.float64)))
            for t in (None, rp.Tune(algo=1))]
     assert err[0] <= err[1]
+
+
+def test_products_that_share_memory():
+    """F over A, which E has read by then."""
+    dims = (96, 64, 96, 96, 50)
+    ni, nj, nk, nl, nm = dims
+    rng = np.random.default_rng(3)
+    mats = [_values("uniform", s, rng) for s in _shapes(dims)]
+    want = _mm3(mats, dims)
+    torch = gu.torch_cuda()
+    a, b, c, d = (gu.dev(m.ravel()) for m in mats)
+    e, g = (torch.zeros(r * k, dtype=torch.float64, device="cuda") for r, k in ((ni, nj), (ni, nl)))
+    rp.check(rp.b200().b200_polybench_3mm(*[t.data_ptr() for t in (a, b, c, d, e, a, g)], *dims,
+                                          None, gu.stream()))
+    assert np.array_equal(gu.host(e).reshape(ni, nj), want[0])
+    assert np.array_equal(gu.host(a)[:nj * nl].reshape(nj, nl), want[1])
+    assert np.array_equal(gu.host(g).reshape(ni, nl), want[2])
