@@ -407,10 +407,10 @@ int b200_polybench_gemm(const double* A, const double* B, double* C, int64_t ni,
 /* E = A*B, F = C*D, G = E*F (FP64)
  *   -- polybench/POLYBENCH_3MM.hpp:61-86, -Cuda.cpp:144-160
  * With inner dimensions from 32 to 4096 the products run on the FP8 tensor
- * cores from 16 exact base-16 digits per value, every element no less accurate
- * than a chain of FP64 FMAs (elements and tiles for which that cannot be told
- * are computed on the FP64 pipe); tune->algo 1 keeps all of it on the FP64
- * pipe, in the suite's order of k.                                          */
+ * cores from 15 base-32 digits per value, every element within 1.25 units of
+ * 2^-53 of itself (elements and tiles for which that cannot be told are
+ * computed on the FP64 pipe); tune->algo 1 keeps all of it on the FP64 pipe, in
+ * the suite's order of k.                                                   */
 int b200_polybench_3mm(const double* A, const double* B, const double* C,
                        const double* D, double* E, double* F, double* G,
                        int64_t ni, int64_t nj, int64_t nk, int64_t nl,

@@ -1,25 +1,29 @@
-// C = A * B in FP64 on the FP8 tensor cores, no less accurate than a chain of
-// FP64 FMAs.
+// C = A * B in FP64 on the FP8 tensor cores, every element as accurate as one
+// rounding of the exact product.
 //
 // GB300's FP64 pipe gives 1.25 TFLOP/s; its e4m3 tensor cores give 4.5 PFLOP/s
 // and, on integers, exact sums.  A value x of a row of A (column of B) whose
-// largest magnitude lies in binade e is cut to a sign and a 64-bit integer in
-// units of 2^(e+1-64), and that into 16 base-16 digits, each with x's sign.
-// The e4m3 code of a digit is the digit itself (codes 0..15 are the linear range
-// 0..15 of 2^-9), so cutting takes masks and byte permutes only.  For every
-// weight w = s + t = 2..17 the digit products A_s * B_t sum to an integer that
-// FP32 holds exactly (at most 16 * 225 * k < 2^24), and the 16 sums combine
-// into one integer and one rounding.
+// largest magnitude lies in binade e is rounded to an integer in units of
+// 2^(e+1-74), and that is cut into 15 balanced base-32 digits -15 .. 16, each
+// with x's sign.  The e4m3 code of a digit is its magnitude (codes 0 .. 16 are the
+// linear range 0 .. 16 of 2^-9) and a sign bit, so cutting takes shifts, masks
+// and byte permutes only.  For every weight w = s + t = 2 .. 17 the digit products
+// A_s * B_t sum to an integer that FP32 holds exactly (at most 15 * 256 * k <
+// 2^24), and the 16 sums combine into one integer and one rounding.
 //
-// Error: what the cuts and the weights from 18 on leave out is below
-// k * 2^-60.2 * 2^(ea+1) * 2^(eb+1); a chain of FMAs errs by up to k * 2^-53 *
-// sum |a||b|.  An element of magnitude at least 2^-7 * 2^(ea+1) * 2^(eb+1) is
-// therefore at least as accurate as a chain's (in fact some ten times more: one
-// rounding instead of k).  The few elements below (one in 1600 for k = 1000
-// uniform values of either sign) are computed again as FP64 dot products; a
-// tile with many of them, or with a row or column that the cut does not take
-// (infinities, NaNs, magnitudes outside 2^-400 .. 2^400), is computed whole on
-// the FP64 pipe.
+// Error: the weights from 18 on leave out at most 108 k units of the combined
+// integer (kDropped), a value that lies more than 21 binades below its row's
+// largest and so lost bits at most 256 (kPerCut).  An element at least 2^55
+// times what may be missing from it is stored: it errs by its one rounding and
+// at most a quarter of 2^-53 of itself, whatever the values, where a chain of
+// FP64 FMAs rounds k times.  The others (one in 30000 for k = 1000 uniform values
+// of either sign) are computed again as FP64 dot products; a tile with many of
+// them, or with a row or column that the cut does not take (infinities, NaNs,
+// magnitudes outside 2^-400 .. 2^400), is computed whole on the FP64 pipe.
+// (16 unsigned base-16 digits, cut off below, took 592 us where this takes 774:
+// 1000 x 1100 x 1010 x 1200 x 1000, but what they left out, of one sign and
+// 2^-60 of the largest products, cost up to 9 bits where one large value of a
+// row met a small one.)
 //
 // A CTA owns a 128 x 32 tile of C: with 16 weights its sums fill tensor memory
 // (16 x 32 FP32 columns), so nothing is folded before the end, and the digits
@@ -29,13 +33,11 @@
 // while one thread issues the MMAs of the other stage.
 //
 // Measured, E = A B, F = C D, G = E F (us, against the FP64 pipe's kernel):
-// 1000 x 1100 x 1010 x 1200 x 1000  590 / 7360, 2048^3 each 3055 / 43600, 500^3
-// 107 / 1630, 250^3 68 / 790, 100^3 55 / 320.  A tile of k = 1000 takes 15 us
-// for its exponents, 60 us for the steps (the cutting is the bound: the MMAs
-// alone take 38 us, at 4.5 PFLOP/s) and 10 us to combine; before, with 16
-// operands' loads in a row and guards on each, the steps took 82 us.  16
-// cutting warps were slower than 8 (639 us), which keep their loads in
-// registers.
+// 1000 x 1100 x 1010 x 1200 x 1000  774 / 7360.  The cutting is the bound (some
+// 46 integer instructions a value), the MMAs alone take 38 us of a tile of
+// k = 1000, at 4.5 PFLOP/s.  Extracting the fields by spreading 20 bits over
+// four bytes of each value took 885 us; two fields of four values at a time,
+// by byte permutes, 774.
 #include "b200_dgemm.cuh"
 #include "b200_f64emu.cuh"
 #include "b200_launch.cuh"
@@ -48,17 +50,20 @@ namespace {
 using namespace tcgen05;
 
 constexpr int TM = 128, TN = 32, KS = 32;     // tile of C, k per step
-constexpr int kDigits = 16;
+constexpr int kDigits = 15, kWeights = 16;
 constexpr int kCutters = 8;                   // warps that cut and, at the end, combine
 constexpr int kThreads = 32 * (1 + kCutters);
 constexpr int kStages = 2;
 constexpr int kQuads = TM / 4 / kCutters;  // quads of A per thread and step
 constexpr uint32_t kATile = TM * 128;                      // four digits: 128 rows x 128 bytes
-constexpr uint32_t kAStage = kATile * (kDigits / 4);       // 64 KB
-constexpr uint32_t kBBytes = kDigits * TN * 128;           // 64 KB: four k steps side by side
+constexpr uint32_t kAStage = kATile * ((kDigits + 3) / 4);   // 64 KB
+constexpr uint32_t kBBytes = kDigits * TN * 128;           // 60 KB: the stages side by side
 constexpr uint32_t kTmemCols = 512;
 constexpr int64_t kMaxK = 4096;
 constexpr int kMaxRedo = 48;                  // elements redone one by one; more: the whole tile
+// Bounds of what a sum leaves out, in its last unit (see above).
+constexpr int kDropped = 108;                 // per k: 256 (13/32 + 12/32^2 + 11/32^3 + ..)
+constexpr int kPerCut = 1 << 8;               // per value that lost bits
 constexpr uint64_t kWaitNs = 1000000000ull;
 
 struct Smem {
@@ -66,12 +71,14 @@ struct Smem {
   uint32_t tmem;
   int abort, bad, redo;
   int ea[TM], eb[TN];        // biased exponents of the rows' and columns' largest values; 0: all zero
+  int cut_a[TM], cut_b[TN];  // how many of their values lost bits
   uint32_t list[kMaxRedo];
 };
 constexpr uint32_t kOperands = kStages * kAStage + kBBytes;
 constexpr size_t kSmemBytes = 1024 + kOperands + sizeof(Smem);
 static_assert(kSmemBytes <= 232448, "shared memory budget");
-static_assert(16 * 225 * kMaxK < (1 << 24), "sums are exact in FP32");
+static_assert(kDigits * 256 * kMaxK < (1 << 24), "sums are exact in FP32");
+static_assert(kWeights * TN <= kTmemCols, "the sums fit in tensor memory");
 
 struct Products {
   Product p[2];
@@ -95,35 +102,88 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t s) {
   return __byte_perm(a, b, s);
 }
 
-// Digits 1 .. 16 (most significant first) of a quad, four values of a row or
-// column: out[d] holds digit d + 1 of all four, as e4m3 codes.
-__device__ __forceinline__ void cut4(const double (&x)[4], int e, uint32_t (&out)[kDigits]) {
-  uint32_t w[4][4];  // odd and even digits of the upper and the lower half
+// 15 in every 5-bit field of 75 bits (32-bit words, the lowest first): added to
+// an integer, it makes the fields the balanced digits -15 .. 16 plus 15.
+constexpr uint32_t kFifteens0 = 0xdef7bdefu, kFifteens1 = 0xf7bdef7bu, kFifteens2 = 0x3deu;
+
+// Two values' bits `at` .. `at` + 9 of a word, side by side in 16 bits each.
+__device__ __forceinline__ uint32_t pair(uint32_t a, uint32_t b, int at) {
+  const uint32_t y = at / 8;
+  return prmt(a, b, y * 0x1111u + 0x5410u) >> (at % 8);
+}
+
+// The e4m3 codes of four digits from their fields (digit + 15 in the low bits
+// of each byte): a digit of magnitude m up to 16 has the code m, with the sign
+// in bit 7.  `flip` holds 0x80 in the bytes of the non-negative values.
+__device__ __forceinline__ uint32_t codes(uint32_t fields, uint32_t flip) {
+  const uint32_t p = (fields >> 4) & 0x01010101u;  // digit > 0
+  const uint32_t m = ((fields & 0x0f0f0f0fu) ^ 0x0f0f0f0fu) ^ (p * 15u);
+  return (p * 0x81u + m) ^ flip;
+}
+
+// A value more than 21 binades below its row's (column's) largest, `below` of
+// them further: its significand in the unit, rounded to nearest.
+__device__ __forceinline__ uint64_t far_below(uint64_t bits, uint32_t below, int* lost) {
+  const uint64_t m = (bits & f64emu::kFrac) | f64emu::kHidden;
+  if ((bits << 1) == 0u) return 0u;
+  uint64_t v = 0;
+  if ((bits << 1 >> 53) != 0u && below <= 54u) v = (m + (1ull << (below - 1u))) >> below;
+  if (v == 0u || v << below != m) atomicAdd(lost, 1);
+  return v;
+}
+
+// Digits 1 .. 15 (most significant first) of a quad, four values of a row or
+// column: out[d] holds digit d + 1 of all four, as e4m3 codes.  `lost` counts
+// the values that lost bits.
+__device__ __forceinline__ void cut4(const double (&x)[4], int e, int* lost,
+                                     uint32_t (&out)[kDigits]) {
+  uint32_t hi[4], mh[4], ml[4];
+  int up[4];  // the significand's shift to the unit 2^(e + 1 - 74)
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
     const uint64_t b = f64emu::bits_opaque(x[m]);
-    const uint32_t hi = static_cast<uint32_t>(b >> 32);
-    const uint32_t d = static_cast<uint32_t>(e) - ((hi >> 20) & 0x7ffu);
-    uint64_t v;  // zero and subnormal values are shifted out
-    asm("shr.u64 %0, %1, %2;"
-        : "=l"(v)
-        : "l"(((b & f64emu::kFrac) | f64emu::kHidden) << 11), "r"(d));
-    const uint32_t sign = static_cast<uint32_t>(static_cast<int32_t>(hi) >> 31) & 0x80808080u;
-    const uint32_t vh = static_cast<uint32_t>(v >> 32), vl = static_cast<uint32_t>(v);
-    w[0][m] = ((vh >> 4) & 0x0f0f0f0fu) | sign;
-    w[1][m] = (vh & 0x0f0f0f0fu) | sign;
-    w[2][m] = ((vl >> 4) & 0x0f0f0f0fu) | sign;
-    w[3][m] = (vl & 0x0f0f0f0fu) | sign;
+    hi[m] = static_cast<uint32_t>(b >> 32);
+    ml[m] = static_cast<uint32_t>(b);
+    mh[m] = (hi[m] & 0xfffffu) | 0x100000u;
+    up[m] = static_cast<int>((hi[m] >> 20) & 0x7ffu) - (e - 21);
   }
+  if (min(min(up[0], up[1]), min(up[2], up[3])) < 0) {
 #pragma unroll
-  for (int h = 0; h < 4; ++h) {  // byte b of the four words side by side
-    const uint32_t a = prmt(w[h][0], w[h][1], 0x5140), c = prmt(w[h][2], w[h][3], 0x5140);
-    const uint32_t p = prmt(w[h][0], w[h][1], 0x7362), q = prmt(w[h][2], w[h][3], 0x7362);
-    const int d = (h >> 1) * 8 + (h & 1);
-    out[d + 6] = prmt(a, c, 0x5410);
-    out[d + 4] = prmt(a, c, 0x7632);
-    out[d + 2] = prmt(p, q, 0x5410);
-    out[d + 0] = prmt(p, q, 0x7632);
+    for (int m = 0; m < 4; ++m) {
+      if (up[m] < 0) {
+        const uint64_t v = far_below(f64emu::bits_opaque(x[m]), static_cast<uint32_t>(-up[m]), lost);
+        mh[m] = static_cast<uint32_t>(v >> 32);
+        ml[m] = static_cast<uint32_t>(v);
+        up[m] = 0;
+      }
+    }
+  }
+  uint32_t t[5][4];  // 75 bits in three words; bits 30 .. 61 and 60 .. 91
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    t[0][m] = __funnelshift_l(0u, ml[m], up[m]);
+    t[1][m] = __funnelshift_l(ml[m], mh[m], up[m]);
+    t[2][m] = __funnelshift_l(mh[m], 0u, up[m]);
+    asm("add.cc.u32 %0, %0, %3;\n\t"
+        "addc.cc.u32 %1, %1, %4;\n\t"
+        "addc.u32 %2, %2, %5;"
+        : "+r"(t[0][m]), "+r"(t[1][m]), "+r"(t[2][m])
+        : "n"(kFifteens0), "n"(kFifteens1), "n"(kFifteens2));
+    t[3][m] = __funnelshift_r(t[0][m], t[1][m], 30);
+    t[4][m] = __funnelshift_r(t[1][m], t[2][m], 28);
+  }
+  // the bytes of a word of codes: values 0, 2, 1, 3 of the quad
+  const uint32_t signs = prmt(prmt(hi[0], hi[2], 0x0073), prmt(hi[1], hi[3], 0x0073), 0x5410);
+  const uint32_t flip = ~signs & 0x80808080u;
+  // two fields at a time: word and bit where they start
+  constexpr int kWord[8] = {0, 0, 0, 3, 1, 1, 4, 2}, kBit[8] = {0, 10, 20, 0, 8, 18, 0, 6};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t* v = t[kWord[j]];
+    const uint32_t a = pair(v[0], v[1], kBit[j]), b = pair(v[2], v[3], kBit[j]);
+    out[kDigits - 1 - 2 * j] = codes((a & 0x00ff00ffu) | ((b << 8) & 0xff00ff00u), flip);
+    if (j < 7)
+      out[kDigits - 2 - 2 * j] = codes(((a >> 5) & 0x00ff00ffu) | ((b << 3) & 0xff00ff00u), flip);
   }
 }
 
@@ -198,8 +258,10 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
     }
     mbar_init(&sm.done, 1);
     sm.abort = sm.bad = sm.redo = 0;
+    for (int i = 0; i < TN; ++i) sm.cut_b[i] = 0;
     mbar_init_fence();
   }
+  if (tid < TM) sm.cut_a[tid] = 0;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&sm.tmem)),
@@ -296,9 +358,9 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
         if (!ok) break;
         tc_fence_after();
         const uint64_t bd = sw128_desc(b_smem) + 2u * s;
-        for (uint32_t d = 0; d < kDigits; ++d) {
+        for (int d = 0; d < kDigits; ++d) {
           const uint64_t ad = sw128_desc(a_smem + s * kAStage + (d >> 2) * kATile) + 2u * (d & 3u);
-          const uint32_t n = TN * (kDigits - d);
+          const uint32_t n = TN * min(kDigits, kWeights - d);
           mma(tmem + TN * d, ad, bd, n < 256u ? n : 256u);
           if (n > 256u) mma(tmem + TN * d + 256u, ad, bd + (256u * 128u >> 4), n - 256u);
         }
@@ -369,7 +431,7 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
       uint32_t out[kDigits];
 #pragma unroll
       for (int u = 0; u < kQuads; ++u) {
-        cut4(v.a[u], ea[u], out);
+        cut4(v.a[u], ea[u], &sm.cut_a[row[u]], out);
         const uint32_t at = a_smem + s * kAStage + row[u] * 128 + (quad & 3) * 4;
 #pragma unroll
         for (int d = 0; d < kDigits; ++d)
@@ -378,7 +440,7 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
                out[d]);
       }
       if (cuts_b) {
-        cut4(v.b, eb, out);
+        cut4(v.b, eb, &sm.cut_b[lane], out);
         const uint32_t at =
             b_smem + lane * 128 + (((s * 2 + (cw >> 2)) ^ (lane & 7)) << 4) + (cw & 3) * 4;
 #pragma unroll
@@ -398,6 +460,7 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
       if (!cut(t, now)) break;
     }
     // ---- combine ----
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kCutters) : "memory");  // cut_a and cut_b are whole
     if (__all_sync(0xffffffffu, mbar_wait(&sm.done, 0u, abort_flag, kWaitNs))) {
       tc_fence_after();
       constexpr int NC = 4 * TN / kCutters;  // columns per thread
@@ -419,26 +482,31 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
           for (int c = 0; c < NC; ++c) {
             const int n = __float2int_rn(__uint_as_float(f[c]) * 262144.0f);
             const int n1 = __float2int_rn(__uint_as_float(f1[c]) * 262144.0f);
-            half[h][c] = half[h][c] * 256 + (n * 16 + n1);
+            half[h][c] = half[h][c] * 1024 + (n * 32 + n1);
           }
         }
       }
       const int64_t i = i0 + r;
       if (i < g.m) {
-        const int e = sm.ea[r];
+        const int e = sm.ea[r], lost = sm.cut_a[r];
+        const int left_out = kDropped * static_cast<int>(g.k);
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
           const int64_t j = j0 + c0 + c;
           if (j < g.n) {
             const int f = sm.eb[c0 + c];
-            // 2^(ea + 1) * 2^(eb + 1) * 16^-17
-            const double unit = f64emu::from_bits(static_cast<uint64_t>(e + f - 1023 + 2 - 68) << 52);
-            const double v = fma(static_cast<double>(half[0][c]), 4294967296.0,
-                                 static_cast<double>(half[1][c]));
-            const uint32_t ve = (static_cast<uint32_t>(__double2hiint(v)) >> 20) & 0x7ffu;
+            // 2^(ea + 2) * 2^(eb + 2) * 32^-17
+            const double unit = f64emu::from_bits(static_cast<uint64_t>(e + f - 1023 + 4 - 85) << 52);
+            const long long low = ((half[0][c] & 0xfffffll) << 40) + half[1][c];
+            const double v = fma(static_cast<double>(half[0][c] >> 20), 0x1p60,
+                                 static_cast<double>(low));
+            const float least = static_cast<float>(left_out + kPerCut * (lost + sm.cut_b[c0 + c]));
+            // the upper word of 2^55 times `least`, rounded up
+            const uint32_t keep =
+                (__float_as_uint(least) >> 3) + ((1023u - 127u + 55u) << 20) + 1u;
             if (e == 0 || f == 0) {
               g.C[i * g.n + j] = 0.0;
-            } else if (ve >= 1023u + 61u) {  // at least 2^-7 of 2^68
+            } else if ((static_cast<uint32_t>(__double2hiint(v)) & 0x7fffffffu) >= keep) {
               g.C[i * g.n + j] = v * unit;
             } else {
               const int at_list = atomicAdd(&sm.redo, 1);
