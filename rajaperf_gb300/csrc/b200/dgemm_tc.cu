@@ -17,13 +17,16 @@
 // times what may be missing from it is stored: it errs by its one rounding and
 // at most a quarter of 2^-53 of itself, whatever the values, where a chain of
 // FP64 FMAs rounds k times.  The others (one in 30000 for k = 1000 uniform values
-// of either sign) are computed again as FP64 dot products; a tile with many of
-// them, or with a row or column that the cut does not take (infinities, NaNs,
-// magnitudes outside 2^-400 .. 2^400), is computed whole on the FP64 pipe.
-// (16 unsigned base-16 digits, cut off below, took 592 us where this takes 774:
-// 1000 x 1100 x 1010 x 1200 x 1000, but what they left out, of one sign and
-// 2^-60 of the largest products, cost up to 9 bits where one large value of a
-// row met a small one.)
+// of either sign) are computed again as FP64 dot products, one by one; a tile with
+// many of them (max_redo), or with a row or column that the cut does not take
+// (infinities, NaNs, magnitudes outside 2^-400 .. 2^400), is computed whole on
+// the FP64 pipe.  Where most elements are like that (a diagonal matrix, say, whose
+// products are mostly zeros), four of them, computed first, tell, and the tile
+// skips the digits (1000^3 each, a diagonal matrix: 6600 us against 7150 without
+// them, and 6120 on the FP64 pipe alone; they take 1.3 % of other calls).
+// (16 unsigned base-16 digits, cut off below, took 508 us where this takes 705,
+// 1000^3 each, but what they left out, of one sign and 2^-60 of the largest
+// products, cost up to 9 bits where one large value of a row met a small one.)
 //
 // A CTA owns a 128 x 32 tile of C: with 16 weights its sums fill tensor memory
 // (16 x 32 FP32 columns), so nothing is folded before the end, and the digits
@@ -33,11 +36,13 @@
 // while one thread issues the MMAs of the other stage.
 //
 // Measured, E = A B, F = C D, G = E F (us, against the FP64 pipe's kernel):
-// 1000 x 1100 x 1010 x 1200 x 1000  774 / 7360.  The cutting is the bound (some
+// 1000 x 1100 x 1010 x 1200 x 1000  787 / 7360; 1000^3 each, uniform, normal,
+// Student-t (3) and log-normal values 705 - 766 / 6120, 500^3 145 / 1560, 250^3 86 /
+// 790, 100^3 50 / 320, 32^3 27 / 113.  The cutting is the bound (some
 // 46 integer instructions a value), the MMAs alone take 38 us of a tile of
 // k = 1000, at 4.5 PFLOP/s.  Extracting the fields by spreading 20 bits over
-// four bytes of each value took 885 us; two fields of four values at a time,
-// by byte permutes, 774.
+// four bytes of each value was 14 % slower than two fields of four values at a
+// time, by byte permutes.
 #include "b200_dgemm.cuh"
 #include "b200_f64emu.cuh"
 #include "b200_launch.cuh"
@@ -60,7 +65,8 @@ constexpr uint32_t kAStage = kATile * ((kDigits + 3) / 4);   // 64 KB
 constexpr uint32_t kBBytes = kDigits * TN * 128;           // 60 KB: the stages side by side
 constexpr uint32_t kTmemCols = 512;
 constexpr int64_t kMaxK = 4096;
-constexpr int kMaxRedo = 48;                  // elements redone one by one; more: the whole tile
+constexpr int kProbes = 4;
+constexpr int kProbesBad = 3;                 // probes that fail before a tile skips the digits
 // Bounds of what a sum leaves out, in its last unit (see above).
 constexpr int kDropped = 108;                 // per k: 256 (13/32 + 12/32^2 + 11/32^3 + ..)
 constexpr int kPerCut = 1 << 8;               // per value that lost bits
@@ -72,7 +78,8 @@ struct Smem {
   int abort, bad, redo;
   int ea[TM], eb[TN];        // biased exponents of the rows' and columns' largest values; 0: all zero
   int cut_a[TM], cut_b[TN];  // how many of their values lost bits
-  uint32_t list[kMaxRedo];
+  double probe[kProbes];     // some of the tile's elements as FP64 dot products
+  uint16_t list[TM * TN];
 };
 constexpr uint32_t kOperands = kStages * kAStage + kBBytes;
 constexpr size_t kSmemBytes = 1024 + kOperands + sizeof(Smem);
@@ -84,6 +91,15 @@ struct Products {
   Product p[2];
   int tiles0;  // tiles of p[0]
 };
+
+// Elements redone one by one; more: the whole tile.  Where the two cost the same
+// (us per tile beyond the digits' pass, an element and the tile): k = 32 0.11 and
+// 47, 100 0.12 and 100, 250 0.22 and 260, 1000 1.0 and 1080, 4000 5 and 4270.
+__device__ __forceinline__ int max_redo(int64_t k) { return k < 100 ? 512 : 896; }
+
+// The row and column of probe p, one in every quarter of the tile's.
+__device__ __forceinline__ int probe_row(int p) { return p * (TM / kProbes + 1); }
+__device__ __forceinline__ int probe_col(int p) { return p * (TN / kProbes); }
 
 // The key of x's magnitude: above zero for any non-zero x, ordered by binade.
 __device__ __forceinline__ uint32_t key(double x) {
@@ -327,6 +343,28 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
     }
     uint32_t* cols = reinterpret_cast<uint32_t*>(base);  // [kCutters][TN], before the operands
     cols[cw * TN + lane] = col;
+  } else {
+    // the probes: kLanes lanes each, 32 loads in flight per lane
+    constexpr int kLanes = 32 / kProbes;
+    const int p = lane / kLanes;
+    const int64_t i = i0 + probe_row(p), j = j0 + probe_col(p);
+    const double* a = g.A + (i < g.m ? i : g.m - 1) * g.k;
+    const double* b = g.B + (j < g.n ? j : g.n - 1);
+    double dot = 0.0;
+    for (int64_t k = lane % kLanes; k < g.k; k += kLanes * 16) {
+      double x[16], y[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        const int64_t ku = k + kLanes * u;
+        x[u] = ku < g.k ? a[ku] : 0.0;
+        y[u] = ku < g.k ? b[ku * g.n] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 16; ++u) dot = fma(x[u], y[u], dot);
+    }
+#pragma unroll
+    for (int off = kLanes / 2; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
+    if (lane % kLanes == 0) sm.probe[p] = dot;
   }
   // the sums start at zero
   if (warp >= 1 && warp <= 4) {  // one warp per quadrant of tensor memory's lanes
@@ -343,6 +381,17 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
     uint32_t all = 0u;
     for (int w = 0; w < kCutters; ++w) all = max(all, cols[w * TN + tid]);
     sm.eb[tid] = exponent(all, &sm.bad);
+    __syncwarp();
+    // how many of the probes would be computed again
+    bool again = false;
+    if (tid < kProbes) {
+      const int e = sm.ea[probe_row(tid)], f = sm.eb[probe_col(tid)];
+      const double least = f64emu::from_bits(
+          static_cast<uint64_t>(e + f - 1023 + 4 - 85 + 55) << 52) * (kDropped * static_cast<double>(g.k));
+      again = e != 0 && f != 0 && fabs(sm.probe[tid]) < least;
+    }
+    const int count = __popc(__ballot_sync(0xffffffffu, again));
+    if (tid == 0 && count >= kProbesBad) sm.bad = 1;
   }
   __syncthreads();
   const uint32_t tmem = sm.tmem;
@@ -510,7 +559,7 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
               g.C[i * g.n + j] = v * unit;
             } else {
               const int at_list = atomicAdd(&sm.redo, 1);
-              if (at_list < kMaxRedo) sm.list[at_list] = static_cast<uint32_t>(r * TN + c0 + c);
+              sm.list[at_list] = static_cast<uint16_t>(r * TN + c0 + c);
             }
           }
         }
@@ -525,7 +574,7 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
                  "r"(kTmemCols)
                  : "memory");
   }
-  whole = whole || sm.abort || sm.redo > kMaxRedo;
+  whole = whole || sm.abort || sm.redo > max_redo(g.k);
   if (whole) {
     fp64_tile(g, i0, j0, base);
     return;
