@@ -2,12 +2,12 @@
 // data[i]): per-bin reductions over a bin index per item.
 //
 // HISTOGRAM: up to 16 bins (the suite's default is 10), each thread counts in
-// packed 8-bit register counters; up to 16384 bins (55000 for
-// long arrays), a CTA counts into a shared-memory histogram, a warp whose items are all of one bin with a single
-// add (the suite's default bin layout is long runs of one bin; combining any
-// equal lanes with __match_any_sync took 90 us where this takes 29, 2^24 items
-// in 50 random bins); the CTA then adds its counts to the global counters with
-// 64-bit atomics.  Integer
+// packed 8-bit register counters; up to 16384 bins (55000 for long arrays), a CTA
+// counts into a shared-memory histogram, lanes of one bin together where a warp
+// holds many of them (kCountTogether: 2^24 items in 50 bins, random bins, one bin
+// in long runs, two in turn, nine tenths in one: 28, 26, 28, 29 us; always
+// together 92, 29, 29, 31; only where all 32 lanes agree 30, 29, 43, 66); the CTA
+// then adds its counts to the global counters with 64-bit atomics.  Integer
 // sums do not depend on order, so the counts are exact.  The global counters
 // start from counts_init (one small copy kernel).
 //
@@ -55,6 +55,14 @@ __global__ void copy_u64_kernel(const unsigned long long* __restrict__ src,
     dst[b] = src[b];
 }
 
+constexpr unsigned int kNoBin = 0xffffffffu;  // the key of an item outside the bins
+
+// An add to shared memory takes a cycle or two per lane that hits the same
+// counter, __match_any_sync a step per bin that the warp's lanes hold: from this
+// many lanes of one bin on (a middle lane's, the likeliest to lie in a run or in
+// a frequent bin) the lanes of a bin are counted together.
+constexpr int kCountTogether = 12;
+
 template <int BS>
 __global__ void __launch_bounds__(BS)
 histogram_shared_kernel(const int64_t* __restrict__ bins, int64_t n, int64_t num_bins,
@@ -74,9 +82,16 @@ histogram_shared_kernel(const int64_t* __restrict__ bins, int64_t n, int64_t num
 #pragma unroll
     for (int u = 0; u < kItems; ++u) {
       const bool ok = b[u] >= 0 && b[u] < num_bins;
-      const unsigned int key = ok ? static_cast<unsigned int>(b[u]) : 0xffffffffu;
-      const bool one_bin = __all_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, 0));
-      if (ok && (!one_bin || lane == 0u)) atomicAdd(&s_cnt[key], one_bin ? 32u : 1u);
+      const unsigned int key = ok ? static_cast<unsigned int>(b[u]) : kNoBin;
+      unsigned int peers = __ballot_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, 16));
+      if (peers == 0xffffffffu) {
+        if (ok && lane == 0u) atomicAdd(&s_cnt[key], 32u);
+      } else if (__popc(peers) >= kCountTogether) {
+        peers = __match_any_sync(0xffffffffu, key);
+        if (ok && lane == __ffs(peers) - 1u) atomicAdd(&s_cnt[key], __popc(peers));
+      } else if (ok) {
+        atomicAdd(&s_cnt[key], 1u);
+      }
     }
   }
   __syncthreads();
@@ -337,8 +352,12 @@ int b200_algorithm_histogram(const int64_t* bins, int64_t n, int64_t num_bins,
         histogram_shared_kernel<1024><<<static_cast<int>(grid), 1024, smem, st>>>(bins, n, num_bins,
                                                                                  counts);
       } else {
-        histogram_shared_kernel<kBlock><<<bin_grid(n), kBlock, smem, st>>>(bins, n, num_bins,
-                                                                           counts);
+        // (2^24 items in 50 bins: 28 us with eight CTAs per SM, 31 with four; in 1000,
+        // where every CTA has more to add to the global bins: 35 and 33)
+        const int64_t grid = std::min<int64_t>(ceil_div(n, kBlock * kItems),
+                                               device_info().sm_count * (num_bins <= 64 ? 8 : 4));
+        histogram_shared_kernel<kBlock><<<static_cast<int>(grid), kBlock, smem, st>>>(
+            bins, n, num_bins, counts);
       }
     } else {
       histogram_global_kernel<<<bin_grid(n) * 4, kBlock, 0, st>>>(bins, n, num_bins, counts);
