@@ -39,7 +39,7 @@ constexpr int64_t kSharedBins = 16384;  // HISTOGRAM: 64 KB of 32-bit counters,
 constexpr int64_t kMaxSharedBins = 55000;  // for 64 items a bin and more 215 KB
 constexpr int64_t kBlockBins = 2048;    // in CTAs of kBlock threads up to here, of 1024 above
 constexpr int64_t kPrivateBins = 96;    // MULTI_REDUCE: 256 x 96 x 8 B = 192 KB
-constexpr int64_t kSharedSums = 28000;  // MULTI_REDUCE: 224 KB of sums
+constexpr int64_t kSharedSums = 28000;  // a multiple of 4; MULTI_REDUCE: 224 KB of sums
 constexpr int kSumThreads = 1024;
 
 int bin_grid(int64_t n) {
@@ -257,51 +257,137 @@ __global__ void multi_reduce_global_kernel(const int64_t* __restrict__ bins,
   }
 }
 
+// The lanes of `rest` (not empty) with one of its lanes' key, the middle one's
+// if it is in there.
+__device__ __forceinline__ unsigned int peers_of(unsigned int key, unsigned int rest) {
+  const int lane = (rest >> 16) & 1u ? 16 : __ffs(rest) - 1;
+  return rest & __ballot_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, lane));
+}
+
 // `copies` sets of the CTA's sums, one for every few warps: an FP64 add to
-// shared memory is a compare-and-swap loop, and warps that share a set make each
-// other repeat it (2^24 items in 97 random bins: 2724 us with global atomics, 449
-// with one set, 103 with 32; in 3000 bins: 306, 97 and 83; in 20000: 182 and 79).  While a warp's items are all of one bin its lanes add them up in
-// registers, and the warp adds their total when the bin changes.
+// shared memory is a compare-and-swap loop, which lanes and warps that hit one
+// bin make each other repeat (2^24 items in 97 random bins: 2724 us with global
+// atomics, 449 with one set, 103 with 32; in 3000 bins: 306, 97 and 83).  A thread
+// takes four consecutive items and adds up neighbours of one bin; lanes whose four
+// items continue the bin of the lane before add up along the warp; and where many
+// lanes of a step still hold one bin, the warp sums them.
+constexpr int kRun = 4;
+// Where a bin's sum lies in a set: the low two bits are turned so that bins 4
+// apart, as the lanes of a step hold them where bins follow each other, fall
+// into different banks (2^24 items over 16384 bins in turn: 82 -> 70 us).
+__host__ __device__ constexpr int sum_at(unsigned int bin) {
+  return static_cast<int>(bin ^ ((bin >> 4) & 3u));
+}
+__host__ __device__ constexpr int sum_set(int num_bins) { return (num_bins + 3) & ~3; }
+constexpr int kRunLanes = 8;      // lanes with neighbours of one bin that make it worth while
+constexpr int kSumTogether = 12;  // lanes of one bin: five adds on the FP64 pipe against as many
+
 __global__ void __launch_bounds__(kSumThreads)
 multi_reduce_shared_kernel(const int64_t* __restrict__ bins, const double* __restrict__ data,
-                           int64_t n, int num_bins, int copies, double* __restrict__ values) {
+                           int64_t n, int num_bins, int copies, bool vec,
+                           double* __restrict__ values) {
   extern __shared__ double s_sum[];
-  for (int b = threadIdx.x; b < copies * num_bins; b += kSumThreads) s_sum[b] = 0.0;
+  const int set = sum_set(num_bins);
+  for (int b = threadIdx.x; b < copies * set; b += kSumThreads) s_sum[b] = 0.0;
   __syncthreads();
+  constexpr unsigned int kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  double* sums = s_sum + (threadIdx.x >> 5) % copies * num_bins;
-  unsigned int run = 0xffffffffu;  // the bin that `acc` belongs to
+  double* sums = s_sum + (threadIdx.x >> 5) % copies * set;
+  unsigned int held = kNoBin;  // the bin of the lanes' `acc`: the warp's last items were all of it
   double acc = 0.0;
   auto flush = [&] {
-    if (run != 0xffffffffu) {
+    if (held != kNoBin) {
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-      if (lane == 0) atomicAdd(&sums[run], acc);
+      for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(kAll, acc, off);
+      if (lane == 0) atomicAdd(&sums[sum_at(held)], acc);
     }
     acc = 0.0;
   };
-  for (int64_t t0 = static_cast<int64_t>(blockIdx.x) * (kSumThreads * kItems); t0 < n;
-       t0 += static_cast<int64_t>(gridDim.x) * (kSumThreads * kItems)) {
-    unsigned int key[kItems];
-    double v[kItems];
+  constexpr int kGroups = kItems / kRun;
+  constexpr int64_t kStep = static_cast<int64_t>(kSumThreads) * kRun;
+  for (int64_t t0 = static_cast<int64_t>(blockIdx.x) * (kGroups * kStep); t0 < n;
+       t0 += static_cast<int64_t>(gridDim.x) * (kGroups * kStep)) {
+    int64_t b[kGroups][kRun];
+    double v[kGroups][kRun];
 #pragma unroll
-    for (int u = 0; u < kItems; ++u) {
-      const int64_t i = t0 + u * kSumThreads + threadIdx.x;
-      const int64_t b = (i < n) ? __ldcs(bins + i) : -1;
-      v[u] = (i < n) ? __ldcs(data + i) : 0.0;
-      key[u] = (b >= 0 && b < num_bins) ? static_cast<unsigned int>(b) : 0xffffffffu;
+    for (int g = 0; g < kGroups; ++g) {
+      const int64_t i = t0 + g * kStep + threadIdx.x * kRun;
+      if (vec && i + kRun <= n) {
+#pragma unroll
+        for (int q = 0; q < kRun; q += 2) {
+          const longlong2 k2 = __ldcs(reinterpret_cast<const longlong2*>(bins + i + q));
+          const double2 v2 = __ldcs(reinterpret_cast<const double2*>(data + i + q));
+          b[g][q] = k2.x;
+          b[g][q + 1] = k2.y;
+          v[g][q] = v2.x;
+          v[g][q + 1] = v2.y;
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < kRun; ++q) {
+          b[g][q] = i + q < n ? __ldcs(bins + i + q) : -1;
+          v[g][q] = i + q < n ? __ldcs(data + i + q) : 0.0;
+        }
+      }
     }
 #pragma unroll
-    for (int u = 0; u < kItems; ++u) {
-      const unsigned int first = __shfl_sync(0xffffffffu, key[u], 0);
-      if (__all_sync(0xffffffffu, key[u] == first)) {
-        if (first != run) {
-          flush();
-          run = first;
+    for (int g = 0; g < kGroups; ++g) {
+      unsigned int key[kRun];
+#pragma unroll
+      for (int q = 0; q < kRun; ++q)
+        key[q] = b[g][q] >= 0 && b[g][q] < num_bins ? static_cast<unsigned int>(b[g][q]) : kNoBin;
+      constexpr int kLast = kRun - 1;
+      bool equal = false, whole = true;  // neighbours in one bin: any, all
+#pragma unroll
+      for (int q = 1; q < kRun; ++q) {
+        equal |= key[q] == key[q - 1];
+        whole &= key[q] == key[q - 1];
+      }
+      const unsigned int step = __ballot_sync(kAll, key[1] != kNoBin);
+      const bool together = step && __popc(peers_of(key[1], step)) >= kSumTogether;
+      if (__popc(__ballot_sync(kAll, equal)) >= kRunLanes) {
+#pragma unroll
+        for (int q = 1; q < kRun; ++q) {
+          if (key[q] == key[q - 1]) {
+            v[g][q] += v[g][q - 1];
+            key[q - 1] = kNoBin;
+          }
         }
-        acc += v[u];
-      } else if (key[u] != 0xffffffffu) {
-        atomicAdd(&sums[key[u]], v[u]);
+        const unsigned int before = __shfl_up_sync(kAll, key[kLast], 1);
+        const unsigned int heads =
+            __ballot_sync(kAll, lane == 0 || !whole || before != key[kLast]);
+        if (heads == 1u && __all_sync(kAll, whole)) {
+          if (key[kLast] != held) {
+            flush();
+            held = key[kLast];
+          }
+          acc += v[g][kLast];
+          continue;
+        }
+        const int start = 31 - __clz(static_cast<int>(heads & (kAll >> (31 - lane))));
+        for (int off = 1; __any_sync(kAll, lane - off >= start); off *= 2) {
+          const double left = __shfl_up_sync(kAll, v[g][kLast], off);
+          if (lane - off >= start) v[g][kLast] += left;
+        }
+        if (lane < 31 && !((heads >> (lane + 1)) & 1u)) key[kLast] = kNoBin;  // added to the next
+      }
+#pragma unroll
+      for (int q = 0; q < kRun; ++q) {
+        bool mine = key[q] != kNoBin;
+        if (together) {
+          unsigned int rest = __ballot_sync(kAll, mine);
+          while (rest) {  // the same in every lane
+            const unsigned int peers = peers_of(key[q], rest);
+            if (__popc(peers) < kSumTogether) break;
+            double sum = (peers >> lane) & 1u ? v[g][q] : 0.0;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(kAll, sum, off);
+            if (lane == __ffs(peers) - 1) atomicAdd(&sums[sum_at(key[q])], sum);
+            rest &= ~peers;
+          }
+          mine = (rest >> lane) & 1u;
+        }
+        if (mine) atomicAdd(&sums[sum_at(key[q])], v[g][q]);
       }
     }
   }
@@ -309,7 +395,7 @@ multi_reduce_shared_kernel(const int64_t* __restrict__ bins, const double* __res
   __syncthreads();
   for (int b = threadIdx.x; b < num_bins; b += kSumThreads) {
     double s = 0.0;
-    for (int c = 0; c < copies; ++c) s += s_sum[c * num_bins + b];
+    for (int c = 0; c < copies; ++c) s += s_sum[c * set + sum_at(b)];
     if (s != 0.0) atomicAdd(&values[b], s);
   }
 }
@@ -382,11 +468,13 @@ int b200_basic_multi_reduce(const int64_t* bins, const double* data, int64_t n,
   cudaStream_t st = as_stream(stream);
   if (num_bins > kPrivateBins || n == 0) {
     copy_f64_kernel<<<small_grid(num_bins), 256, 0, st>>>(values_init, values, num_bins);
-    // each CTA clears and adds all its sums: from 256 items a bin on (2^20 items in
-    // 3000 bins: 22 us against 25 with global atomics)
-    if (n >= (1 << 18) && num_bins <= kSharedSums && n >= 256 * num_bins) {
-      const int copies = static_cast<int>(std::min<int64_t>(32, kSharedSums / num_bins));
-      const size_t smem = static_cast<size_t>(copies * num_bins) * sizeof(double);
+    // each CTA clears and adds all its sums: from 350 items a bin on (random bins,
+    // against global atomics: 2^20 items in 2049 bins 22 us and 33; 2^18 in 1000 bins
+    // 22 and 18)
+    if (n >= (1 << 18) && num_bins <= kSharedSums && n >= 350 * num_bins) {
+      const int set = sum_set(static_cast<int>(num_bins));
+      const int copies = std::min<int>(32, static_cast<int>(kSharedSums) / set);
+      const size_t smem = static_cast<size_t>(copies * set) * sizeof(double);
       const int rc = allow_dynamic_smem(
           reinterpret_cast<const void*>(multi_reduce_shared_kernel), smem,
           "b200_basic_multi_reduce");
@@ -395,7 +483,8 @@ int b200_basic_multi_reduce(const int64_t* bins, const double* data, int64_t n,
       const int64_t grid = std::min<int64_t>(ceil_div(n, kSumThreads * kItems),
                                              fit * device_info().sm_count);
       multi_reduce_shared_kernel<<<static_cast<int>(grid), kSumThreads, smem, st>>>(
-          bins, data, n, static_cast<int>(num_bins), copies, values);
+          bins, data, n, static_cast<int>(num_bins), copies, aligned16(bins) && aligned16(data),
+          values);
     } else if (n > 0)
       multi_reduce_global_kernel<<<bin_grid(n) * 4, kBlock, 0, st>>>(bins, data, n, num_bins,
                                                                       values);

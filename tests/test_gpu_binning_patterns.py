@@ -96,7 +96,8 @@ def _time(call):
 
 
 @pytest.mark.parametrize("which,kind,factor", [
-    (0, "two", 1.25), (0, "20", 1.25), (0, "frequent", 1.35)])
+    (0, "two", 1.25), (0, "20", 1.25), (0, "frequent", 1.35),
+    (1, "8", 1.25), (1, "20", 1.5)])
 def test_few_bins_in_a_warp_cost_little(which, kind, factor):
     n, nb = 1 << 24, 16384
     rng = np.random.default_rng(3)
