@@ -242,11 +242,18 @@ heat3d_step(const double* __restrict__ S, double* __restrict__ D, int64_t N, int
 // stay on the FP64 pipe: four register-operand FMAs per point (2 a and 0.125 x
 // are exact factors) where the kernel above issues 6.5; every FULL-th row also
 // runs direction k in fixed point, one FMA left.  Results are bit for bit the
-// suite's; a thread that met a value outside its window redoes its points on
-// the FP64 pipe after the loop.  One column and 64 registers per thread: two or
-// four columns save unpacking but leave too few warps to hide the loads.  Per
-// half-step (with the overlapped launches): 188 -> 108 us at 256^3 (FP64 pipe
-// and integer ALU both near 90%), 19.4 -> 11.1 us at 98^3, 8.3 -> 2.5 us at 32^3.
+// suite's.  A walk shares one window, taken anew after eight rows if the column's
+// values have moved; a thread that met a value outside it computes its rows again,
+// each in a window of its own and all of direction k on the FP64 pipe, and on the
+// FP64 pipe alone what does not fit there either.  One column and 64 registers
+// per thread: two or four columns save unpacking but leave too few warps to hide
+// the loads (as does more state in the walk: the rows' own windows there, 80
+// registers, 126 us).  Per half-step (with the overlapped launches), against the
+// kernel above, uniform values: 188 -> 107 us at 256^3 (FP64 pipe and integer
+// ALU both near 90%), 14.8 -> 8.5 us at 98^3, 7.9 -> 2.5 us at 34^3; fields that
+// leave a window, 256^3: exp(-400 r^2) 259 -> 224, exp(60 y) 534 -> 154, a
+// product of sines 230 -> 198 (435, 445 and 348 with one window per walk and
+// all its rows again on the FP64 pipe).
 template <int PJ, int FULL>
 __global__ void __launch_bounds__(256)
 heat3d_fix(const double* S, double* D, int64_t N, int zero) {
@@ -267,49 +274,69 @@ heat3d_fix(const double* S, double* D, int64_t N, int zero) {
   // row j's neighbours in k and i
   double a = ld(p), an = ld(p + N), kp = ld(p + 1), km = ld(p - 1);
   double ip = ld(p + NN), im = ld(p - NN);
-  const Unit u = unit_at(a, 4, slow);
+  Unit u = unit_at(a, 3, slow);
   int64_t fp = fix(ld(p - N), u, slow), fa = fix(a, u, slow);  // rows j - 1, j
+  constexpr int kShare = 8;  // rows
+  for (int r0 = 0; r0 < rows; r0 += kShare) {
+    if (r0 > 0 && (static_cast<uint32_t>(__double2hiint(a)) >> 20) - u.low - 2u > 3u) {
+      u = unit_at(a, 3, slow);
+      fp = fix(ld(p - N), u, slow);
+      fa = fix(a, u, slow);
+    }
+    const int end = PJ > kShare ? min(rows, r0 + kShare) : rows;
 #pragma unroll FULL
-  for (int r = 0; r < rows; ++r) {
-    double an2, kp2, km2, ip2, im2;
-    if (r + 1 < rows) {
-      an2 = ld(p + 2 * N);
-      kp2 = ld(p + N + 1);
-      km2 = ld(p + N - 1);
-      ip2 = ld(p + N + NN);
-      im2 = ld(p + N - NN);
+    for (int r = r0; r < end; ++r) {
+      double an2, kp2, km2, ip2, im2;
+      if (r + 1 < rows) {
+        an2 = ld(p + 2 * N);
+        kp2 = ld(p + N + 1);
+        km2 = ld(p + N - 1);
+        ip2 = ld(p + N + NN);
+        im2 = ld(p + N - NN);
+      }
+      const int64_t fn = fix(an, u, slow);
+      const int64_t two = 2 * fa;
+      const int64_t ti = round53(round53(fix(ip, u, slow) - two) + fix(im, u, slow));
+      const int64_t tj = round53(round53(fn - two) + fp);
+      double t;
+      if (r % FULL == FULL - 1) {
+        const int64_t tk = round53(round53(fix(kp, u, slow) - two) + fix(km, u, slow));
+        t = pack(round53(ti + tj) + tk, u, -3);
+      } else {
+        const double tk = fform::add(fma(a, mtwo, kp), km, fr);
+        t = fma(tk, eighth, pack(ti + tj, u, -3));
+      }
+      *q = fform::add(t, a, fr);
+      a = an;
+      an = an2;
+      kp = kp2;
+      km = km2;
+      ip = ip2;
+      im = im2;
+      fp = fa;
+      fa = fn;
+      p += N;
+      q += N;
     }
-    const int64_t fn = fix(an, u, slow);
-    const int64_t two = 2 * fa;
-    const int64_t ti = round53(round53(fix(ip, u, slow) - two) + fix(im, u, slow));
-    const int64_t tj = round53(round53(fn - two) + fp);
-    double t;
-    if (r % FULL == FULL - 1) {
-      const int64_t tk = round53(round53(fix(kp, u, slow) - two) + fix(km, u, slow));
-      t = pack(round53(ti + tj) + tk, u, -3);
-    } else {
-      const double tk = fform::add(fma(a, mtwo, kp), km, fr);
-      t = fma(tk, eighth, pack(ti + tj, u, -3));
-    }
-    *q = fform::add(t, a, fr);
-    a = an;
-    an = an2;
-    kp = kp2;
-    km = km2;
-    ip = ip2;
-    im = im2;
-    fp = fa;
-    fa = fn;
-    p += N;
-    q += N;
   }
   if (slow) {
-    for (int r = 0; r < rows; ++r) {
-      const int64_t c = k + N * (j0 + r + N * i);
-      const double a0 = ld(S + c);
-      D[c] = 0.125 * (ld(S + c + NN) - 2.0 * a0 + ld(S + c - NN)) +
-             0.125 * (ld(S + c + N) - 2.0 * a0 + ld(S + c - N)) +
-             0.125 * (ld(S + c + 1) - 2.0 * a0 + ld(S + c - 1)) + a0;
+    p = S + k + N * (j0 + N * i);
+    q = D + k + N * (j0 + N * i);
+    for (int r = 0; r < rows; ++r, p += N, q += N) {
+      const double c = ld(p), i1 = ld(p + NN), i0 = ld(p - NN), j1 = ld(p + N), jm = ld(p - N);
+      const double k1 = ld(p + 1), k0 = ld(p - 1);
+      bool out = false;
+      const Unit w = unit_at(c, 3, out);
+      const int64_t two = 2 * fix(c, w, out);
+      const int64_t ti = round53(round53(fix(i1, w, out) - two) + fix(i0, w, out));
+      const int64_t tj = round53(round53(fix(j1, w, out) - two) + fix(jm, w, out));
+      const double tk = fform::add(fma(c, mtwo, k1), k0, fr);
+      double v = fform::add(fma(tk, eighth, pack(ti + tj, w, -3)), c, fr);
+      if (__any_sync(__activemask(), out) && out)
+        // contracted as the kernel above has the suite's expression
+        v = fma(0.125, fma(-2.0, c, k1) + k0,
+                fma(0.125, fma(-2.0, c, i1) + i0, 0.125 * (fma(-2.0, c, j1) + jm))) + c;
+      *q = v;
     }
   }
 }
