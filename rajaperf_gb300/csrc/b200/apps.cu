@@ -252,7 +252,7 @@ vol3d_walk(const Vol3D p, int64_t n, int zero) {
                    fma(a[0], b[1], -fform::mul(a[1], b[0], fr))};
     };
     auto dot = [&](const double (&s)[3], const Cross& w) {
-      return fma(s[2], w.z, fma(s[1], w.y, fform::mul(s[0], w.x, fr)));
+      return fma(s[2], w.z, fma(s[0], w.x, fform::mul(s[1], w.y, fr)));
     };
     const Cross w2 = cross(d74, d60);
     double v = dot(s1, cross(d72, d30));
