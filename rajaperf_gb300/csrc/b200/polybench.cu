@@ -465,10 +465,13 @@ fdtd2d_step_fused(double* __restrict__ ex, double* __restrict__ ey, double* __re
   double* sHzFirst = s_fdtd + TH * (kFdtdCols + 1) + (TH + 1) * kFdtdCols;
   double* sHzLast = sHzFirst + TH;
 
-  t += begin();
+  // every index below is made from t, bx or by: no load moves ahead of the wait
+  const unsigned int z = begin();
+  t += z;
   const int tid = threadIdx.x % kFdtdCols, lane = tid & 31;
   const int group = threadIdx.x / kFdtdCols, first = group * (TH / G);
-  const int64_t bx = blockIdx.x, by = blockIdx.y;
+  const int64_t bx = static_cast<int64_t>(blockIdx.x) + z;
+  const int64_t by = static_cast<int64_t>(blockIdx.y) + z;
   const int64_t j0 = bx * kFdtdCols, i0 = by * TH;
   const int64_t j = j0 + tid;
   const int rows = static_cast<int>(nx - i0 < TH ? nx - i0 : TH);
