@@ -8,9 +8,9 @@
 // 53 leading bits (round53) gives what the FP64 pipe's add would, in about 13
 // instructions, and only the last sum is packed into a double again.
 //
-// Range: values of one sign whose exponents lie in a window of 8 binades fit
-// exactly as magnitudes (f < 2^60), so sums of up to 7 of them stay below
-// 2^63 - 2^10.  A value outside the window or of the other sign (zeros, subnormals,
+// Range: values of one sign whose exponents lie in a window of 7 (8) binades fit
+// exactly as magnitudes (f < 2^59 or 2^60), so sums of up to 15 (7) of them stay
+// below 2^63 - 2^10.  A value outside the window or of the other sign (zeros, subnormals,
 // infinities and NaNs among them) sets `slow`, and the caller redoes the point
 // on the FP64 pipe.  The unit is kept far from both ends of the exponent
 // range, so no intermediate result is subnormal or overflows, and a zero sum
@@ -28,7 +28,7 @@ struct Unit {
   uint32_t low;
 };
 
-// The window of 8 binades that starts `below` binades under x's.
+// The window that starts `below` binades under x's.
 __device__ __forceinline__ Unit unit_at(double x, int below, bool& slow) {
   const uint32_t e = static_cast<uint32_t>(__double2hiint(x)) >> 20;
   const uint32_t low = e - static_cast<uint32_t>(below);
@@ -36,10 +36,15 @@ __device__ __forceinline__ Unit unit_at(double x, int below, bool& slow) {
   return Unit{low};
 }
 
+// x in the unit; BINADES: the window's.  Eight serve HEAT_3D, which sums six
+// values; the test for seven is the cheaper one (JACOBI_2D 529 us a pass at
+// 1002^2 and 40 steps, with eight 538).
+template <uint32_t BINADES = 7>
 __device__ __forceinline__ int64_t fix(double x, Unit u, bool& slow) {
+  static_assert(BINADES == 7 || BINADES == 8, "sums of what its callers add fit in 63 bits");
   const uint64_t b = f64emu::bits_opaque(x);
   const uint32_t s = (static_cast<uint32_t>(b >> 32) >> 20) - u.low;
-  slow |= s > 7u;
+  slow |= s > BINADES - 1u;
   int64_t m;
   asm("shl.b64 %0, %1, %2;" : "=l"(m) : "l"((b & f64emu::kFrac) | f64emu::kHidden), "r"(s));
   return m;

@@ -275,13 +275,13 @@ heat3d_fix(const double* S, double* D, int64_t N, int zero) {
   double a = ld(p), an = ld(p + N), kp = ld(p + 1), km = ld(p - 1);
   double ip = ld(p + NN), im = ld(p - NN);
   Unit u = unit_at(a, 3, slow);
-  int64_t fp = fix(ld(p - N), u, slow), fa = fix(a, u, slow);  // rows j - 1, j
+  int64_t fp = fix<8>(ld(p - N), u, slow), fa = fix<8>(a, u, slow);  // rows j - 1, j
   constexpr int kShare = 8;  // rows
   for (int r0 = 0; r0 < rows; r0 += kShare) {
     if (r0 > 0 && (static_cast<uint32_t>(__double2hiint(a)) >> 20) - u.low - 2u > 3u) {
       u = unit_at(a, 3, slow);
-      fp = fix(ld(p - N), u, slow);
-      fa = fix(a, u, slow);
+      fp = fix<8>(ld(p - N), u, slow);
+      fa = fix<8>(a, u, slow);
     }
     const int end = PJ > kShare ? min(rows, r0 + kShare) : rows;
 #pragma unroll FULL
@@ -294,13 +294,13 @@ heat3d_fix(const double* S, double* D, int64_t N, int zero) {
         ip2 = ld(p + N + NN);
         im2 = ld(p + N - NN);
       }
-      const int64_t fn = fix(an, u, slow);
+      const int64_t fn = fix<8>(an, u, slow);
       const int64_t two = 2 * fa;
-      const int64_t ti = round53(round53(fix(ip, u, slow) - two) + fix(im, u, slow));
+      const int64_t ti = round53(round53(fix<8>(ip, u, slow) - two) + fix<8>(im, u, slow));
       const int64_t tj = round53(round53(fn - two) + fp);
       double t;
       if (r % FULL == FULL - 1) {
-        const int64_t tk = round53(round53(fix(kp, u, slow) - two) + fix(km, u, slow));
+        const int64_t tk = round53(round53(fix<8>(kp, u, slow) - two) + fix<8>(km, u, slow));
         t = pack(round53(ti + tj) + tk, u, -3);
       } else {
         const double tk = fform::add(fma(a, mtwo, kp), km, fr);
@@ -327,9 +327,9 @@ heat3d_fix(const double* S, double* D, int64_t N, int zero) {
       const double k1 = ld(p + 1), k0 = ld(p - 1);
       bool out = false;
       const Unit w = unit_at(c, 3, out);
-      const int64_t two = 2 * fix(c, w, out);
-      const int64_t ti = round53(round53(fix(i1, w, out) - two) + fix(i0, w, out));
-      const int64_t tj = round53(round53(fix(j1, w, out) - two) + fix(jm, w, out));
+      const int64_t two = 2 * fix<8>(c, w, out);
+      const int64_t ti = round53(round53(fix<8>(i1, w, out) - two) + fix<8>(i0, w, out));
+      const int64_t tj = round53(round53(fix<8>(j1, w, out) - two) + fix<8>(jm, w, out));
       const double tk = fform::add(fma(c, mtwo, k1), k0, fr);
       double v = fform::add(fma(tk, eighth, pack(ti + tj, w, -3)), c, fr);
       if (__any_sync(__activemask(), out) && out)
