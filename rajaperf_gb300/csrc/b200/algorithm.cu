@@ -227,7 +227,7 @@ scan_pipelined(const T* x, T* y, int64_t n, T init, unsigned int tiles, ScanHead
     sm.fail_prefix = 0;
     mbar_init_fence();
   }
-  const unsigned int z = begin();
+  const unsigned int z = begin_early();
   x += z;
   hdr += z;
   descs += z;
@@ -485,7 +485,7 @@ scan_pipelined_f64(const double* x, double* y, int64_t n, double init, unsigned 
     }
     mbar_init_fence();
   }
-  const unsigned int z = begin();
+  const unsigned int z = begin_early();
   x += z;
   hdr += z;
   descs += z;

@@ -2,12 +2,24 @@
 //
 // A kernel launched in a stream behind another one normally starts some 2.2 us
 // after it has drained (measured on GB300: dependent DAXPYs of 4096, 1M and
-// 4M elements take 4.10, 6.15 and 12.3 us each).  launch() asks for the
-// grid to be set up while its predecessor still runs, and begin() is the
-// device side: it lets the successor be set up in turn, then waits until every
-// preceding grid has completed and its writes are visible (1.79, 3.63 and
-// 9.93 us each).  In a CUDA graph the edge between two such nodes becomes a
-// programmatic one (1.95 -> 1.74 and 3.79 -> 3.58 us a node).
+// 4M elements take 4.23, 6.23 and 12.4 us each).  launch() asks for the
+// grid to be set up as its predecessor's CTAs end, and begin() is the
+// device side: it waits until every preceding grid has completed and its writes
+// are visible (1.47, 3.57 and 9.4 us each).  In a CUDA graph the edge between
+// two such nodes becomes a programmatic one (1.80 -> 1.28 and 3.81 -> 3.32 us a node).
+//
+// The successor's CTAs are placed as slots fall free.  Letting that begin earlier,
+// at this grid's own start, gains nothing and loses where neither grid fills the
+// chip: the CTAs go to the SMs that this grid left emptier, or that ended first,
+// and wait there, two or three on one SM and none on the next.  A call in a graph
+// (us; set up after the predecessor, at its start, as its CTAs end): FDTD_2D, 8
+// steps of 500^2, 57.3, 85.6, 53.5; HYDRO_2D 200^2 6.9, 9.9, 6.1; REDUCE_SUM of
+// 700001 7.2, 9.8, 6.9; VOL3D 50^3 14.9, 17.8, 14.5; the 1-D kernels at 4096 and
+// 200000 elements, 14 calls, 40.6, 34.3, 32.4 and 67.9, 72.7, 62.3.  A persistent
+// kernel whose CTAs have an SM to themselves has no such loss, and its successor
+// gains from the earlier start (INDEXLIST, 3M items, 17.3, 13.3, 14.3 us):
+// begin_early().  (So would, by less than 1 %, grids of many waves, but a test of
+// the grid's size in every thread costs more: JACOBI_2D at 1002^2 526 -> 539 us.)
 //
 // Rules for a kernel that is launched by launch():
 //  * every thread calls begin() before its first access to global memory, so
@@ -28,18 +40,22 @@
 
 namespace b200 {
 
-// Lets the next grid of the stream be set up, waits for the preceding ones;
-// returns 0.
+// Waits for the preceding grids of the stream; returns 0.
 __device__ __forceinline__ unsigned int begin() {
   unsigned int zero;
   asm volatile(
-      "griddepcontrol.launch_dependents;\n\t"
       "griddepcontrol.wait;\n\t"
       "mov.u32 %0, 0;"
       : "=r"(zero)
       :
       : "memory");
   return zero;
+}
+
+// The same, and lets the next grid be set up at once.
+__device__ __forceinline__ unsigned int begin_early() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  return begin();
 }
 
 // kernel<<<grid, block, smem, st>>>(args...) with the overlap above; launch

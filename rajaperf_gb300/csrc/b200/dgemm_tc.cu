@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  int tile = static_cast<int>(begin()) + static_cast<int>(blockIdx.x);
+  int tile = static_cast<int>(begin_early()) + static_cast<int>(blockIdx.x);
   const bool second = tile >= ps.tiles0;
   Product g = second ? ps.p[1] : ps.p[0];
   if (second) tile -= ps.tiles0;

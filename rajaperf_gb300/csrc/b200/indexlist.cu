@@ -230,7 +230,7 @@ indexlist_pipelined(const double* x, int32_t* list, int64_t n, int64_t* len, uns
     for (int g = 0; g < kGroups; ++g) sm.fail_ballot[g] = sm.fail_writer[g] = 0;
     mbar_init_fence();
   }
-  const unsigned int z = begin();
+  const unsigned int z = begin_early();
   x += z;
   hdr += z;
   descs += z;
