@@ -474,12 +474,6 @@ int b200_apps_vol3d(const double* x, const double* y, const double* z, double* v
   return launch_map1d("b200_apps_vol3d", f, n, tune, as_stream(stream));
 }
 
-// DEL_DOT_VEC_2D's corner sums opened on the integer pipes by default.
-// Measured on GB300 (the bench's 4096^2 jittered mesh, 256 x 2): none 0.927
-// ms, 2: 0.908, 4: 0.892, 6: 0.829, all 8: 1.068 (the integer pipes, which
-// also carry the two divisions and five products, become the bound).
-constexpr int kDelDotIntAdds = 6;
-
 int b200_apps_del_dot_vec_2d(const double* x, const double* y, const double* xdot,
                              const double* ydot, double* div,
                              const int64_t* real_zones, int64_t n_real_zones,
@@ -490,7 +484,11 @@ int b200_apps_del_dot_vec_2d(const double* x, const double* y, const double* xdo
     return invalid("b200_apps_del_dot_vec_2d: bad args");
   // two zones per thread by default: 1.3% faster than four at 4096^2 zones;
   // tune->tile_z = 1 + corner sums opened on the integer pipes (0, 2, 4, 6
-  // or 8; 2, 4 and 8 with 256 threads x 2 zones)
+  // or 8; 2, 4 and 8 with 256 threads x 2 zones); measured on the bench's 4096^2
+  // jittered mesh, 256 x 2, before the launches overlapped: none 0.927 ms, 2:
+  // 0.908, 4: 0.892, 6: 0.829, all 8: 1.068 (the integer pipes, which also
+  // carry the two divisions and five products, become the bound); the default,
+  // fixed point, 0.69
   if (half == 0.5) {
     const int kd = (tune && tune->tile_z) ? tune->tile_z - 1 : 0;
     // the variants with integer-pipe adds run the default shape (256 x 2)

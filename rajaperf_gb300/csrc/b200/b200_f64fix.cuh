@@ -5,7 +5,7 @@
 // similar size, again and again: here a value is unpacked once, into a 64-bit
 // integer in a unit of the thread's own (`Unit`, from one of its values'
 // exponents), and an add of two such integers is exact; rounding the sum to its
-// 53 leading bits (round53) gives what the FP64 pipe's add would, in about 13
+// 53 leading bits (round53) gives what the FP64 pipe's add would, in about 11
 // instructions, and only the last sum is packed into a double again.
 //
 // Range: values of one sign whose exponents lie in a window of 7 (8) binades fit

@@ -438,11 +438,11 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
       const int64_t i = i0 + row[u] < g.m ? i0 + row[u] : g.m - 1;
       ap[u] = g.A + i * g.k + quad;
     }
-    // the first eight warps also cut a quad of B each: k = cw, column `lane`
-    const bool cuts_b = cw < 8;
+    // each warp also cuts a quad of B: k = cw, column `lane`
+    static_assert(kCutters == KS / 4, "a quad of B per warp");
     const int eb = sm.eb[lane] ? sm.eb[lane] : 1023;
     const int64_t j = j0 + lane < g.n ? j0 + lane : g.n - 1;
-    const double* bp = g.B + (cw & 7) * g.n + j;
+    const double* bp = g.B + cw * g.n + j;
     const int64_t b8 = 8 * g.n;
     struct Values {
       double a[kQuads][4], b[4];
@@ -454,17 +454,15 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
         for (int u = 0; u < kQuads; ++u)
 #pragma unroll
           for (int m = 0; m < 4; ++m) v.a[u][m] = ap[u][8 * m];
-        if (cuts_b) {
 #pragma unroll
-          for (int m = 0; m < 4; ++m) v.b[m] = bp[m * b8];
-        }
+        for (int m = 0; m < 4; ++m) v.b[m] = bp[m * b8];
       } else {
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
           const int64_t k = k0 + 8 * m;
 #pragma unroll
           for (int u = 0; u < kQuads; ++u) v.a[u][m] = k + quad < g.k ? ap[u][8 * m] : 0.0;
-          v.b[m] = k + (cw & 7) < g.k ? bp[m * b8] : 0.0;
+          v.b[m] = k + cw < g.k ? bp[m * b8] : 0.0;
         }
       }
 #pragma unroll
@@ -488,13 +486,11 @@ __global__ void __launch_bounds__(kThreads, 1) dgemm_tc_kernel(const Products ps
                    ((((d & 3) * 2 + (quad >> 2)) ^ (row[u] & 7)) << 4),
                out[d]);
       }
-      if (cuts_b) {
-        cut4(v.b, eb, &sm.cut_b[lane], out);
-        const uint32_t at =
-            b_smem + lane * 128 + (((s * 2 + (cw >> 2)) ^ (lane & 7)) << 4) + (cw & 3) * 4;
+      cut4(v.b, eb, &sm.cut_b[lane], out);
+      const uint32_t bt =
+          b_smem + lane * 128 + (((s * 2 + (cw >> 2)) ^ (lane & 7)) << 4) + (cw & 3) * 4;
 #pragma unroll
-        for (int d = 0; d < kDigits; ++d) st32(at + d * TN * 128, out[d]);
-      }
+      for (int d = 0; d < kDigits; ++d) st32(bt + d * TN * 128, out[d]);
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.full[s]);

@@ -173,8 +173,8 @@ static_assert(kEnds + kDraw < kSlots, "end markers fit in the slots");
 static_assert(kRows <= 32, "a lane holds one row's ballots");
 
 // Per-slot state of the tiles between their draw and their list writes
-// (with the ring's limit_ns and abort, for ring::wait and
-// ring::publish_aggregate).
+// (with the ring's kStages, limit_ns and abort, for ring::wait and
+// ring::fetch_prefixes).
 struct Slots {
   using AccT = long long;
   static constexpr int kStages = kSlots;
