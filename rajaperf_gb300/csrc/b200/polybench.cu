@@ -245,7 +245,7 @@ heat3d_step(const double* __restrict__ S, double* __restrict__ D, int64_t N, int
 // suite's.  A walk shares one window, taken anew after eight rows if the column's
 // values have moved; a thread that met a value outside it computes its rows again,
 // each in a window of its own and all of direction k on the FP64 pipe, and on the
-// FP64 pipe alone what does not fit there either.  One column and 64 registers
+// FP64 pipe alone what does not fit there either.  One column and 56 registers
 // per thread: two or four columns save unpacking but leave too few warps to hide
 // the loads (as does more state in the walk: the rows' own windows there, 80
 // registers, 126 us).  Per half-step (with the overlapped launches), against the
