@@ -1081,7 +1081,7 @@ ozaki_tc_paired_kernel(const __grid_constant__ CUtensorMap tmA,
 // 2 .. 8 are exact in 53 bits, 9 and 10 are rounded in place (f64fix::round53),
 // and 11 as the sum is packed, or by an FP64 FMA where the sum is too long.
 // One chunk only: k <= kChunkK.
-// Whole call, against the paired engine (us): 3500 x 3500 x 4200  1892 / 2738
+// Whole call, against the paired engine (us): 3500 x 3500 x 4200  1960 - 2000 / 2758
 // (the slicing, now on the integer pipes, is 135 us less of each),
 // 8192^3 16660 / 22030, 1000^3 131 / 199, 250 x 300 x 400  65 / 170.  A tile of
 // k = 4200 takes 103 us of MMAs (the rate's floor is 92) and 12 us to fold; with
